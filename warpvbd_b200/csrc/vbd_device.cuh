@@ -64,6 +64,7 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 // Elastic gradient / Hessian of one (vertex, tet) slot, accumulated into g, h
 // (h = h00 h01 h02 h11 h12 h22).  d* = u_n - u_v of the tet's other three
 // vertices, q* = (b_n, p): p0 = V*mu, p1 = V*lambda (material-adjusted).
+// fp32 arithmetic; fp64 uses slot_accumulate64 below.
 // ---------------------------------------------------------------------------
 template <typename Real, int MAT>
 __device__ __forceinline__ void slot_accumulate(Real d0x, Real d0y, Real d0z, Real d1x, Real d1y,
@@ -84,51 +85,6 @@ __device__ __forceinline__ void slot_accumulate(Real d0x, Real d0y, Real d0z, Re
   const Real bz = -(q0.z + q1.z + q2.z);
   const Real p0 = q0.w, p1 = q1.w;
   const Real bb = bx * bx + by * by + bz * bz;
-  if (MAT == kSNH && sizeof(Real) == 8) {
-    // fp64: the reference's own form (vbd_solver.py:111-114, 118-123)
-    //   P b = mu' (1 - 1/(Ic+1)) F b + lambda' (J - alpha) cof(F) b
-    // with lambda' (J - alpha) = lambda' (J - 1) - 3/4 mu'.  The difference
-    // J - 1 cancels at small strain, as the reference's J - alpha does; in
-    // double precision that costs ~1e-16 / strain relative, far below the
-    // solver's tolerance, and it needs fewer operations and live values than
-    // the cancellation-free form the fp32 path uses below.
-    const Real F00 = Real(1) + G00, F11 = Real(1) + G11, F22 = Real(1) + G22;
-    const Real Fbx = F00 * bx + G01 * by + G02 * bz;
-    const Real Fby = G10 * bx + F11 * by + G12 * bz;
-    const Real Fbz = G20 * bx + G21 * by + F22 * bz;
-    const Real Ic = F00 * F00 + G01 * G01 + G02 * G02 + G10 * G10 + F11 * F11 + G12 * G12 +
-                    G20 * G20 + G21 * G21 + F22 * F22;
-    // cof(F) row by row: J from row 0, cof(F) b from all three
-    Real c0 = F11 * F22 - G12 * G21, c1 = G12 * G20 - G10 * F22, c2 = G10 * G21 - F11 * G20;
-    const Real J = F00 * c0 + G01 * c1 + G02 * c2;
-    const Real Cbx = c0 * bx + c1 * by + c2 * bz;
-    c0 = G21 * G02 - F22 * G01;
-    c1 = F22 * F00 - G20 * G02;
-    c2 = G20 * G01 - G21 * F00;
-    const Real Cby = c0 * bx + c1 * by + c2 * bz;
-    c0 = G01 * G12 - G02 * F11;
-    c1 = G02 * G10 - F00 * G12;
-    c2 = F00 * F11 - G01 * G10;
-    const Real Cbz = c0 * bx + c1 * by + c2 * bz;
-    const Real p0 = q0.w, p1 = q1.w;
-    const Real inv = Real(1) / (Ic + Real(1));
-    const Real a = p0 * (Real(1) - inv);
-    const Real kJ = p1 * (J - Real(1)) - Real(0.75) * p0;
-    g[0] += a * Fbx + kJ * Cbx;
-    g[1] += a * Fby + kJ * Cby;
-    g[2] += a * Fbz + kJ * Cbz;
-    const Real hF = Real(2) * p0 * inv * inv;
-    const Real hI = a * bb;
-    const Real Fx = hF * Fbx, Fy = hF * Fby, Fz = hF * Fbz;
-    const Real Cx = p1 * Cbx, Cy = p1 * Cby, Cz = p1 * Cbz;
-    h[0] += Fx * Fbx + Cx * Cbx + hI;
-    h[1] += Fx * Fby + Cx * Cby;
-    h[2] += Fx * Fbz + Cx * Cbz;
-    h[3] += Fy * Fby + Cy * Cby + hI;
-    h[4] += Fy * Fbz + Cy * Cbz;
-    h[5] += Fz * Fbz + Cz * Cbz + hI;
-    return;
-  }
   const Real Gbx = G00 * bx + G01 * by + G02 * bz;
   const Real Gby = G10 * bx + G11 * by + G12 * bz;
   const Real Gbz = G20 * bx + G21 * by + G22 * bz;
@@ -214,6 +170,262 @@ __device__ __forceinline__ void slot_accumulate(Real d0x, Real d0y, Real d0z, Re
   }
 }
 
+// ---------------------------------------------------------------------------
+// fp64 slots.  The record table holds one record per distinct tet (not per
+// slot): the rows b_0, b_1, b_2 of its Dm^-1 as double4, with p0, p1, p0 in
+// their fourth values.  A slot names the tet's other vertices n0, n1, n2 in
+// the tet's order and its own place a among the four, and
+//   G = sum over i < 3 of (u_i - u_3) b_i^T
+// needs only those rows: for a = 3 the neighbours are vertices 0, 1, 2, else
+// n2 is vertex 3 and the vertex itself takes row a.  Four slots share a record
+// that way, which is what lets the table of a voxel mesh stay in shared memory
+// (rounding of the rest positions makes hundreds of distinct tets; 635 on the
+// 6,755-tet mass-spring: 61 KB, against 237 KB for its 2,470 slot records).
+// ---------------------------------------------------------------------------
+struct TetRows {
+  double4 r0, r1, r2;  // the rows of n0, n1 and of the remaining vertex below 3
+  double p0, p1;
+};
+
+template <typename Real>
+struct RecTab;
+template <>
+struct RecTab<float> {
+  const float4* p;  // three float4 per slot record, global or shared memory
+};
+template <>
+struct RecTab<double> {
+  const double4* g;        // global memory, three double4 per record
+  const unsigned char* s;  // the copy staged in shared memory, or null
+};
+
+// One aligned 32-byte read-only load.
+__device__ __forceinline__ double4 ldg_row(const double4* p) {
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+      : "l"(p));
+  return v;
+}
+
+// The staged copy swaps the 16-byte halves of every row of records 4-7 mod 8:
+// a record is 96 bytes, so without it the same half of eight consecutive
+// records would fall into four of the eight 16-byte bank groups (70 instead of
+// 50 shared-memory wavefronts per 32 slots on the 11^3 mass-spring).
+__device__ __forceinline__ void stage_table(unsigned char* dst, const RecTab<double>& t, int nrec) {
+  for (int i = threadIdx.x; i < 3 * nrec; i += blockDim.x) {
+    const double4 v = ldg_row(t.g + i);
+    double2* d = reinterpret_cast<double2*>(dst) + 2 * i;
+    const int sw = (i / 3 >> 2) & 1;
+    d[sw] = make_double2(v.x, v.y);
+    d[sw ^ 1] = make_double2(v.z, v.w);
+  }
+}
+__device__ __forceinline__ void stage_table(unsigned char* dst, const RecTab<float>& t, int nrec) {
+  float4* d = reinterpret_cast<float4*>(dst);
+  for (int i = threadIdx.x; i < 3 * nrec; i += blockDim.x) d[i] = ldg4(t.p + i);
+}
+__device__ __forceinline__ RecTab<double> staged(RecTab<double> t, const unsigned char* s) {
+  t.s = s;
+  return t;
+}
+__device__ __forceinline__ RecTab<float> staged(RecTab<float> t, const unsigned char* s) {
+  t.p = reinterpret_cast<const float4*>(s);
+  return t;
+}
+template <typename Real>
+__device__ __forceinline__ RecTab<Real> global_table(const void* tab, int rbase);
+template <>
+__device__ __forceinline__ RecTab<float> global_table<float>(const void* tab, int rbase) {
+  return {reinterpret_cast<const float4*>(tab) + 3 * (size_t)rbase};
+}
+template <>
+__device__ __forceinline__ RecTab<double> global_table<double>(const void* tab, int rbase) {
+  return {reinterpret_cast<const double4*>(tab) + 3 * (size_t)rbase, nullptr};
+}
+
+// The record id and the vertex's place in the tet of an fp64 slot.
+__device__ __forceinline__ int slot_record(int w) { return w >> 2; }
+__device__ __forceinline__ int slot_place(int w) { return w & 3; }
+
+__device__ __forceinline__ TetRows load_rows(const RecTab<double>& t, int w) {
+  const int rec = slot_record(w), a = slot_place(w);
+  const int i0 = a == 0 ? 1 : 0, i1 = a < 2 ? 2 : 1, i2 = a < 2 ? a : 2;
+  TetRows r;
+  if (t.s) {
+    const unsigned char* b = t.s + 96 * rec;
+    const int lo = (rec & 4) << 2, hi = lo ^ 16;
+    auto row = [&](int i) {
+      const double2 x = *reinterpret_cast<const double2*>(b + 32 * i + lo);
+      const double2 y = *reinterpret_cast<const double2*>(b + 32 * i + hi);
+      return make_double4(x.x, x.y, y.x, y.y);
+    };
+    r.r0 = row(i0);
+    r.r1 = row(i1);
+    r.r2 = row(i2);
+  } else {
+    const double4* g = t.g + 3 * (size_t)rec;
+    r.r0 = ldg_row(g + i0);
+    r.r1 = ldg_row(g + i1);
+    r.r2 = ldg_row(g + i2);
+  }
+  // (i0, i1, i2) = (1, 2, 0), (0, 2, 1), (0, 1, 2), (0, 1, 2); row 1 holds p1
+  r.p0 = a == 0 ? r.r1.w : r.r0.w;
+  r.p1 = a == 0 ? r.r0.w : (a == 1 ? r.r2.w : r.r1.w);
+  return r;
+}
+
+// The fp64 vertex update is written with explicit fused multiply-adds: which
+// product of a sum the compiler fuses may differ between two kernels, and every
+// launch shape has to give an environment the same bits.
+__device__ __forceinline__ double dot3(double a0, double b0, double a1, double b1, double a2,
+                                       double b2) {
+  return fma(a2, b2, fma(a1, b1, a0 * b0));
+}
+__device__ __forceinline__ double cross2(double a, double b, double c, double d) {  // ab - cd
+  return fma(a, b, -(c * d));
+}
+
+// Displacement gradient of an fp64 slot: uo the vertex's own displacement,
+// n0, n1, n2 its neighbours'.
+__device__ __forceinline__ void slot_gradient64(const double4& uo, const double4& n0,
+                                                const double4& n1, const double4& n2, int a,
+                                                const TetRows& t, double (&G)[9]) {
+  const bool last = a == 3;  // the vertex is the tet's vertex 3
+  const double bx = last ? uo.x : n2.x, by = last ? uo.y : n2.y, bz = last ? uo.z : n2.z;
+  const double ex = uo.x - n2.x, ey = uo.y - n2.y, ez = uo.z - n2.z;
+  const double d2x = last ? -ex : ex, d2y = last ? -ey : ey, d2z = last ? -ez : ez;
+  const double d0x = n0.x - bx, d0y = n0.y - by, d0z = n0.z - bz;
+  const double d1x = n1.x - bx, d1y = n1.y - by, d1z = n1.z - bz;
+  G[0] = dot3(d0x, t.r0.x, d1x, t.r1.x, d2x, t.r2.x);
+  G[1] = dot3(d0x, t.r0.y, d1x, t.r1.y, d2x, t.r2.y);
+  G[2] = dot3(d0x, t.r0.z, d1x, t.r1.z, d2x, t.r2.z);
+  G[3] = dot3(d0y, t.r0.x, d1y, t.r1.x, d2y, t.r2.x);
+  G[4] = dot3(d0y, t.r0.y, d1y, t.r1.y, d2y, t.r2.y);
+  G[5] = dot3(d0y, t.r0.z, d1y, t.r1.z, d2y, t.r2.z);
+  G[6] = dot3(d0z, t.r0.x, d1z, t.r1.x, d2z, t.r2.x);
+  G[7] = dot3(d0z, t.r0.y, d1z, t.r1.y, d2z, t.r2.y);
+  G[8] = dot3(d0z, t.r0.z, d1z, t.r1.z, d2z, t.r2.z);
+}
+
+// 1 / x for x >= 1: the hardware's approximation and two Newton steps
+// y (2 - x y), each of which doubles its correct bits.
+__device__ __forceinline__ double reciprocal64(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// As slot_accumulate, in fp64; the multiples of the identity in the Hessian
+// go to hI (added to its diagonal once per vertex).
+template <int MAT>
+__device__ __forceinline__ void slot_accumulate64(const double4& uo, const double4& n0,
+                                                  const double4& n1, const double4& n2, int a,
+                                                  const TetRows& t, double (&g)[3], double (&h)[6],
+                                                  double& hI) {
+  double G[9];
+  slot_gradient64(uo, n0, n1, n2, a, t, G);
+  // the vertex's own gradient: row a, or minus the sum of the rows
+  const bool last = a == 3;
+  const double sx = t.r0.x + t.r1.x + t.r2.x, sy = t.r0.y + t.r1.y + t.r2.y,
+               sz = t.r0.z + t.r1.z + t.r2.z;
+  const double bx = last ? -sx : t.r2.x, by = last ? -sy : t.r2.y, bz = last ? -sz : t.r2.z;
+  const double bb = dot3(bx, bx, by, by, bz, bz);
+  if (MAT == kSNH) {
+    // the reference's own form (vbd_solver.py:111-114, 118-123)
+    //   P b = mu' (1 - 1/(Ic+1)) F b + lambda' (J - alpha) cof(F) b
+    // with lambda' (J - alpha) = lambda' (J - 1) - 3/4 mu'.  The difference
+    // J - 1 cancels at small strain, as the reference's J - alpha does; in
+    // double precision that costs ~1e-16 / strain relative, far below the
+    // solver's tolerance, and it needs fewer operations and live values than
+    // the cancellation-free form of the fp32 path.
+    const double F00 = 1.0 + G[0], F11 = 1.0 + G[4], F22 = 1.0 + G[8];
+    const double F01 = G[1], F02 = G[2], F10 = G[3], F12 = G[5], F20 = G[6], F21 = G[7];
+    const double Fbx = dot3(F00, bx, F01, by, F02, bz);
+    const double Fby = dot3(F10, bx, F11, by, F12, bz);
+    const double Fbz = dot3(F20, bx, F21, by, F22, bz);
+    const double Ic = dot3(F00, F00, F01, F01, F02, F02) + dot3(F10, F10, F11, F11, F12, F12) +
+                      dot3(F20, F20, F21, F21, F22, F22);
+    // the columns of cof(F) are cross products of F's columns f0, f1, f2:
+    //   cof(F) b = bx (f1 x f2) + f0 x (bz f1 - by f2),  J = f0 . (f1 x f2)
+    const double cx = cross2(F11, F22, F21, F12), cy = cross2(F21, F02, F01, F22),
+                 cz = cross2(F01, F12, F11, F02);
+    const double J = dot3(F00, cx, F10, cy, F20, cz);
+    const double wx = cross2(bz, F01, by, F02), wy = cross2(bz, F11, by, F12),
+                 wz = cross2(bz, F21, by, F22);
+    const double Cbx = fma(bx, cx, cross2(F10, wz, F20, wy));
+    const double Cby = fma(bx, cy, cross2(F20, wx, F00, wz));
+    const double Cbz = fma(bx, cz, cross2(F00, wy, F10, wx));
+    const double inv = reciprocal64(Ic + 1.0);
+    const double ka = t.p0 * (1.0 - inv);
+    const double kJ = fma(t.p1, J - 1.0, -0.75 * t.p0);
+    g[0] = fma(kJ, Cbx, fma(ka, Fbx, g[0]));
+    g[1] = fma(kJ, Cby, fma(ka, Fby, g[1]));
+    g[2] = fma(kJ, Cbz, fma(ka, Fbz, g[2]));
+    const double hF = 2.0 * t.p0 * (inv * inv);
+    const double Fx = hF * Fbx, Fy = hF * Fby, Fz = hF * Fbz;
+    const double Cx = t.p1 * Cbx, Cy = t.p1 * Cby, Cz = t.p1 * Cbz;
+    h[0] = fma(Cx, Cbx, fma(Fx, Fbx, h[0]));
+    h[1] = fma(Cx, Cby, fma(Fx, Fby, h[1]));
+    h[2] = fma(Cx, Cbz, fma(Fx, Fbz, h[2]));
+    h[3] = fma(Cy, Cby, fma(Fy, Fby, h[3]));
+    h[4] = fma(Cy, Cbz, fma(Fy, Fbz, h[4]));
+    h[5] = fma(Cz, Cbz, fma(Fz, Fbz, h[5]));
+    hI = fma(ka, bb, hI);
+  } else {
+    // E = (G + G^T + G^T G) / 2
+    const double E00 = fma(0.5, dot3(G[0], G[0], G[3], G[3], G[6], G[6]), G[0]);
+    const double E11 = fma(0.5, dot3(G[1], G[1], G[4], G[4], G[7], G[7]), G[4]);
+    const double E22 = fma(0.5, dot3(G[2], G[2], G[5], G[5], G[8], G[8]), G[8]);
+    const double E01 = 0.5 * (G[1] + G[3] + dot3(G[0], G[1], G[3], G[4], G[6], G[7]));
+    const double E02 = 0.5 * (G[2] + G[6] + dot3(G[0], G[2], G[3], G[5], G[6], G[8]));
+    const double E12 = 0.5 * (G[5] + G[7] + dot3(G[1], G[2], G[4], G[5], G[7], G[8]));
+    const double trE = E00 + E11 + E22;
+    const double Ebx = dot3(E00, bx, E01, by, E02, bz);
+    const double Eby = dot3(E01, bx, E11, by, E12, bz);
+    const double Ebz = dot3(E02, bx, E12, by, E22, bz);
+    const double FEbx = Ebx + dot3(G[0], Ebx, G[1], Eby, G[2], Ebz);
+    const double FEby = Eby + dot3(G[3], Ebx, G[4], Eby, G[5], Ebz);
+    const double FEbz = Ebz + dot3(G[6], Ebx, G[7], Eby, G[8], Ebz);
+    const double Fbx = bx + dot3(G[0], bx, G[1], by, G[2], bz);
+    const double Fby = by + dot3(G[3], bx, G[4], by, G[5], bz);
+    const double Fbz = bz + dot3(G[6], bx, G[7], by, G[8], bz);
+    const double k2 = 2.0 * t.p0, kt = t.p1 * trE;
+    g[0] = fma(kt, Fbx, fma(k2, FEbx, g[0]));
+    g[1] = fma(kt, Fby, fma(k2, FEby, g[1]));
+    g[2] = fma(kt, Fbz, fma(k2, FEbz, g[2]));
+    const double bEb = dot3(bx, Ebx, by, Eby, bz, Ebz);
+    // F F^T = I + G + G^T + G G^T; its identity goes to hI
+    const double A00 = fma(2.0, G[0], dot3(G[0], G[0], G[1], G[1], G[2], G[2]));
+    const double A11 = fma(2.0, G[4], dot3(G[3], G[3], G[4], G[4], G[5], G[5]));
+    const double A22 = fma(2.0, G[8], dot3(G[6], G[6], G[7], G[7], G[8], G[8]));
+    const double A01 = G[1] + G[3] + dot3(G[0], G[3], G[1], G[4], G[2], G[5]);
+    const double A02 = G[2] + G[6] + dot3(G[0], G[6], G[1], G[7], G[2], G[8]);
+    const double A12 = G[5] + G[7] + dot3(G[3], G[6], G[4], G[7], G[5], G[8]);
+    const double kff = t.p1 + t.p0;
+    const double kA = t.p0 * bb;
+    const double Kx = kff * Fbx, Ky = kff * Fby, Kz = kff * Fbz;
+    h[0] = fma(kA, A00, fma(Kx, Fbx, h[0]));
+    h[1] = fma(kA, A01, fma(Kx, Fby, h[1]));
+    h[2] = fma(kA, A02, fma(Kx, Fbz, h[2]));
+    h[3] = fma(kA, A11, fma(Ky, Fby, h[3]));
+    h[4] = fma(kA, A12, fma(Ky, Fbz, h[4]));
+    h[5] = fma(kA, A22, fma(Kz, Fbz, h[5]));
+    hI += fma(k2, bEb, fma(kt, bb, kA));
+  }
+}
+
+// Adds the identity part of the Hessian (fp64 slots keep it apart).
+template <typename Real>
+__device__ __forceinline__ void add_identity(Real (&h)[6], Real hI) {
+  if constexpr (sizeof(Real) == 8) {
+    h[0] += hI;
+    h[3] += hI;
+    h[5] += hI;
+  }
+}
+
 // Guarded Newton step: solve H dx = -g by 3x3 Cholesky (the reference's
 // tile_cholesky / tile_cholesky_solve, vbd_solver.py:267-268).  Returns false
 // when a pivot is not positive (H not positive definite).
@@ -236,6 +448,27 @@ __device__ __forceinline__ bool chol_solve3(const Real* h, const Real* g, Real* 
   x[1] = (y1 - L21 * x[2]) * i1;
   x[0] = (y0 - L10 * x[1] - L20 * x[2]) * i0;
   return (h[0] > Real(0)) && (d1 > Real(0)) && (d2 > Real(0));
+}
+
+// The same step in fp64 by cofactors: H^-1 = adj(H) / det(H), one reciprocal
+// where the Cholesky form chains three square roots and three divides, which
+// one lane per vertex runs while the warp waits.  H is positive definite when
+// its leading minors are positive.  Determinants near the ends of the double
+// range take the Cholesky form.
+__device__ __forceinline__ bool solve3(const double* h, const double* g, double* x) {
+  const double c00 = cross2(h[3], h[5], h[4], h[4]), c01 = cross2(h[2], h[4], h[1], h[5]),
+               c02 = cross2(h[1], h[4], h[2], h[3]), c11 = cross2(h[0], h[5], h[2], h[2]),
+               c12 = cross2(h[1], h[2], h[0], h[4]), c22 = cross2(h[0], h[3], h[1], h[1]);
+  const double det = dot3(h[0], c00, h[1], c01, h[2], c02);
+  if (!(fabs(det) > 1e-250 && fabs(det) < 1e250)) return chol_solve3<double>(h, g, x);
+  const double r = -1.0 / det;
+  x[0] = dot3(c00, g[0], c01, g[1], c02, g[2]) * r;
+  x[1] = dot3(c01, g[0], c11, g[1], c12, g[2]) * r;
+  x[2] = dot3(c02, g[0], c12, g[1], c22, g[2]) * r;
+  return (h[0] > 0.0) && (c22 > 0.0) && (det > 0.0);
+}
+__device__ __forceinline__ bool solve3(const float* h, const float* g, float* x) {
+  return chol_solve3<float>(h, g, x);
 }
 
 struct StepConst {
@@ -337,6 +570,33 @@ struct RawSlot<kFmtIdx32> {
 #define VBD_CHECK_BOUNDS 0
 #endif
 
+// One slot of either precision, accumulated into g, h and (fp64) hI: id = the
+// three neighbours and the record, uo = the vertex's own displacement.
+template <typename Real, int MAT, class State, typename S4>
+__device__ __forceinline__ void slot_visit(const State& st, const S4& uo, const int4& id,
+                                           const RecTab<Real>& tab, Real (&g)[3], Real (&h)[6],
+                                           Real& hI) {
+  if constexpr (sizeof(Real) == 8) {
+    const TetRows t = load_rows(tab, id.w);
+    const S4 a = st.load(id.x), b = st.load(id.y), c = st.load(id.z);
+    slot_accumulate64<MAT>(uo, a, b, c, slot_place(id.w), t, g, h, hI);
+  } else {
+    const float4* t = tab.p + 3 * (size_t)id.w;
+    const float4 q0 = t[0], q1 = t[1], q2 = t[2];
+    const S4 a = st.load(id.x), b = st.load(id.y), c = st.load(id.z);
+    // neighbour offsets formed in the state precision, then rounded
+    slot_accumulate<Real, MAT>(Real(a.x - uo.x), Real(a.y - uo.y), Real(a.z - uo.z),
+                               Real(b.x - uo.x), Real(b.y - uo.y), Real(b.z - uo.z),
+                               Real(c.x - uo.x), Real(c.y - uo.y), Real(c.z - uo.z), q0, q1, q2, g,
+                               h);
+  }
+}
+
+template <typename Real>
+__device__ __forceinline__ int record_of(int w) {
+  return sizeof(Real) == 8 ? slot_record(w) : w;
+}
+
 // Slot steps of a chunk whose indices are loaded up front: enough for the
 // reference's 20 incident tets per vertex (MAX_ELEMENTS_PER_VERTEX); longer
 // chunks stream the rest.
@@ -357,17 +617,29 @@ __device__ __forceinline__ void finish_vertex(const DevMesh& m, int gv, int lv,
   using S4 = real4<SReal>;
   const Real mdt2 = Real(tt.w * SReal(sc.inv_dt2));
   Real G[3], H[6];
-  G[0] = g[0] + mdt2 * Real(uo.x - tt.x);
-  G[1] = g[1] + mdt2 * Real(uo.y - tt.y);
-  G[2] = g[2] + mdt2 * Real(uo.z - tt.z);
+  if constexpr (sizeof(Real) == 8) {
+    G[0] = fma(mdt2, uo.x - tt.x, g[0]);
+    G[1] = fma(mdt2, uo.y - tt.y, g[1]);
+    G[2] = fma(mdt2, uo.z - tt.z, g[2]);
+  } else {
+    G[0] = g[0] + mdt2 * Real(uo.x - tt.x);
+    G[1] = g[1] + mdt2 * Real(uo.y - tt.y);
+    G[2] = g[2] + mdt2 * Real(uo.z - tt.z);
+  }
   if (sc.damp) {
     // Rayleigh-like damping kd * H_el (x - x_prev) / dt (vbd_solver.py:222-223)
     const S4 u0 = ldcg4(reinterpret_cast<const S4*>(m.up) + gv);
     const Real kd = Real(sc.kd_dt);
     const Real ex = Real(uo.x - u0.x), ey = Real(uo.y - u0.y), ez = Real(uo.z - u0.z);
-    G[0] += kd * (h[0] * ex + h[1] * ey + h[2] * ez);
-    G[1] += kd * (h[1] * ex + h[3] * ey + h[4] * ez);
-    G[2] += kd * (h[2] * ex + h[4] * ey + h[5] * ez);
+    if constexpr (sizeof(Real) == 8) {
+      G[0] = fma(kd, dot3(h[0], ex, h[1], ey, h[2], ez), G[0]);
+      G[1] = fma(kd, dot3(h[1], ex, h[3], ey, h[4], ez), G[1]);
+      G[2] = fma(kd, dot3(h[2], ex, h[4], ey, h[5], ez), G[2]);
+    } else {
+      G[0] += kd * (h[0] * ex + h[1] * ey + h[2] * ez);
+      G[1] += kd * (h[1] * ex + h[3] * ey + h[4] * ez);
+      G[2] += kd * (h[2] * ex + h[4] * ey + h[5] * ez);
+    }
 #pragma unroll
     for (int i = 0; i < 6; ++i) h[i] *= (Real(1) + kd);
   }
@@ -378,7 +650,7 @@ __device__ __forceinline__ void finish_vertex(const DevMesh& m, int gv, int lv,
   H[4] = h[4];
   H[5] = h[5] + mdt2;
   Real dx[3];
-  if (!chol_solve3<Real>(H, G, dx)) {
+  if (!solve3(H, G, dx)) {
     stat |= kStatGuard;
     if (!sc.strict) {
       // fallback: inertia-only Hessian (m/dt^2) I; a massless vertex stays
@@ -412,9 +684,8 @@ template <typename Real, typename SReal, int TPV, int MAT, int FMT, class State>
 __device__ __forceinline__ void process_chunk(const DevMesh& m, int vbase, const ColorInfo& ci,
                                               int q, int lane, const State& st,
                                               const StepConst& sc, unsigned long long& cmax,
-                                              unsigned& stat, const real4<Real>* tab,
+                                              unsigned& stat, const RecTab<Real>& tab,
                                               unsigned long long* dxrec = nullptr) {
-  using R4 = real4<Real>;
   using S4 = real4<SReal>;
   constexpr int CPW = 32 / TPV;
   const int vi = lane / TPV, sub = lane % TPV;
@@ -455,34 +726,24 @@ __device__ __forceinline__ void process_chunk(const DevMesh& m, int vbase, const
   }
   Real g[3] = {Real(0), Real(0), Real(0)};
   Real h[6] = {Real(0), Real(0), Real(0), Real(0), Real(0), Real(0)};
-  // the environment's record table: shared memory (staged by the caller) or
-  // global memory, read through the same generic pointer
+  Real hI = Real(0);
   auto visit = [&](const int4& id) {
 #if VBD_CHECK_BOUNDS
     if ((unsigned)id.x >= (unsigned)eb.nv || (unsigned)id.y >= (unsigned)eb.nv ||
-        (unsigned)id.z >= (unsigned)eb.nv || (unsigned)id.w >= (unsigned)eb.nrec) {
+        (unsigned)id.z >= (unsigned)eb.nv ||
+        (unsigned)record_of<Real>(id.w) >= (unsigned)eb.nrec) {
       stat |= kStatBounds;
       return;
     }
 #endif
-    const R4* t = tab + 3 * (size_t)id.w;
-    const R4 q0 = t[0];
-    const R4 q1 = t[1];
-    const R4 q2 = t[2];
-    const S4 a = st.load(id.x);
-    const S4 b = st.load(id.y);
-    const S4 c = st.load(id.z);
-    // neighbour offsets formed in the state precision, then rounded
-    slot_accumulate<Real, MAT>(Real(a.x - uo.x), Real(a.y - uo.y), Real(a.z - uo.z),
-                               Real(b.x - uo.x), Real(b.y - uo.y), Real(b.z - uo.z),
-                               Real(c.x - uo.x), Real(c.y - uo.y), Real(c.z - uo.z), q0, q1, q2,
-                               g, h);
+    slot_visit<Real, MAT>(st, uo, id, tab, g, h, hI);
   };
 #pragma unroll
   for (int s = 0; s < PF; ++s)
     if (s < ch.steps && s * TPV + sub < k) visit(RS::unpack(sl[s]));
   for (int s = PF; s < ch.steps; ++s)
     if (s * TPV + sub < k) visit(load_slot<FMT>(m, base + (size_t)s * 32));
+  add_identity(h, hI);
 #pragma unroll
   for (int off = TPV / 2; off > 0; off >>= 1) {
 #pragma unroll
@@ -527,9 +788,8 @@ template <typename Real, typename SReal, int TPV, int MAT, int FMT, class State>
 __device__ __forceinline__ void process_chunk_part(const DevMesh& m, int vbase,
                                                    const ColorInfo& ci, int q, int lane,
                                                    const State& st, unsigned& stat,
-                                                   const real4<Real>* tab, int part, int W,
+                                                   const RecTab<Real>& tab, int part, int W,
                                                    Real* buf) {
-  using R4 = real4<Real>;
   using S4 = real4<SReal>;
   constexpr int CPW = 32 / TPV;
   const int vi = lane / TPV, sub = lane % TPV;
@@ -554,28 +814,21 @@ __device__ __forceinline__ void process_chunk_part(const DevMesh& m, int vbase,
   }
   Real g[3] = {Real(0), Real(0), Real(0)};
   Real h[6] = {Real(0), Real(0), Real(0), Real(0), Real(0), Real(0)};
+  Real hI = Real(0);
   for (int s = part; s < ch.steps; s += W) {
     if (s * TPV + sub >= k) continue;
     const int4 id = load_slot<FMT>(m, base + (size_t)s * 32);
 #if VBD_CHECK_BOUNDS
     if ((unsigned)id.x >= (unsigned)eb.nv || (unsigned)id.y >= (unsigned)eb.nv ||
-        (unsigned)id.z >= (unsigned)eb.nv || (unsigned)id.w >= (unsigned)eb.nrec) {
+        (unsigned)id.z >= (unsigned)eb.nv ||
+        (unsigned)record_of<Real>(id.w) >= (unsigned)eb.nrec) {
       stat |= kStatBounds;
       continue;
     }
 #endif
-    const R4* t = tab + 3 * (size_t)id.w;
-    const R4 q0 = t[0];
-    const R4 q1 = t[1];
-    const R4 q2 = t[2];
-    const S4 a = st.load(id.x);
-    const S4 b = st.load(id.y);
-    const S4 c = st.load(id.z);
-    slot_accumulate<Real, MAT>(Real(a.x - uo.x), Real(a.y - uo.y), Real(a.z - uo.z),
-                               Real(b.x - uo.x), Real(b.y - uo.y), Real(b.z - uo.z),
-                               Real(c.x - uo.x), Real(c.y - uo.y), Real(c.z - uo.z), q0, q1, q2,
-                               g, h);
+    slot_visit<Real, MAT>(st, uo, id, tab, g, h, hI);
   }
+  add_identity(h, hI);
 #pragma unroll
   for (int off = TPV / 2; off > 0; off >>= 1) {
 #pragma unroll
@@ -639,20 +892,8 @@ __device__ __forceinline__ void finish_split_chunk(const DevMesh& m, int vbase,
 // compare two configurations, so constants cancel.
 // ---------------------------------------------------------------------------
 template <typename Real, int MAT>
-__device__ __forceinline__ Real slot_psi(Real d0x, Real d0y, Real d0z, Real d1x, Real d1y,
-                                         Real d1z, Real d2x, Real d2y, Real d2z,
-                                         const real4<Real>& q0, const real4<Real>& q1,
-                                         const real4<Real>& q2) {
-  const Real G00 = d0x * q0.x + d1x * q1.x + d2x * q2.x;
-  const Real G01 = d0x * q0.y + d1x * q1.y + d2x * q2.y;
-  const Real G02 = d0x * q0.z + d1x * q1.z + d2x * q2.z;
-  const Real G10 = d0y * q0.x + d1y * q1.x + d2y * q2.x;
-  const Real G11 = d0y * q0.y + d1y * q1.y + d2y * q2.y;
-  const Real G12 = d0y * q0.z + d1y * q1.z + d2y * q2.z;
-  const Real G20 = d0z * q0.x + d1z * q1.x + d2z * q2.x;
-  const Real G21 = d0z * q0.y + d1z * q1.y + d2z * q2.y;
-  const Real G22 = d0z * q0.z + d1z * q1.z + d2z * q2.z;
-  const Real p0 = q0.w, p1 = q1.w;
+__device__ __forceinline__ Real psi_of(Real G00, Real G01, Real G02, Real G10, Real G11, Real G12,
+                                       Real G20, Real G21, Real G22, Real p0, Real p1) {
   const Real t = G00 + G11 + G22;
   Real psi;
   if (MAT == kSNH) {
@@ -683,6 +924,41 @@ __device__ __forceinline__ Real slot_psi(Real d0x, Real d0y, Real d0z, Real d1x,
   return psi;
 }
 
+template <typename Real, int MAT>
+__device__ __forceinline__ Real slot_psi(Real d0x, Real d0y, Real d0z, Real d1x, Real d1y,
+                                         Real d1z, Real d2x, Real d2y, Real d2z,
+                                         const real4<Real>& q0, const real4<Real>& q1,
+                                         const real4<Real>& q2) {
+  const Real G00 = d0x * q0.x + d1x * q1.x + d2x * q2.x;
+  const Real G01 = d0x * q0.y + d1x * q1.y + d2x * q2.y;
+  const Real G02 = d0x * q0.z + d1x * q1.z + d2x * q2.z;
+  const Real G10 = d0y * q0.x + d1y * q1.x + d2y * q2.x;
+  const Real G11 = d0y * q0.y + d1y * q1.y + d2y * q2.y;
+  const Real G12 = d0y * q0.z + d1y * q1.z + d2y * q2.z;
+  const Real G20 = d0z * q0.x + d1z * q1.x + d2z * q2.x;
+  const Real G21 = d0z * q0.y + d1z * q1.y + d2z * q2.y;
+  const Real G22 = d0z * q0.z + d1z * q1.z + d2z * q2.z;
+  return psi_of<Real, MAT>(G00, G01, G02, G10, G11, G12, G20, G21, G22, q0.w, q1.w);
+}
+
+// slot_psi of one slot of either precision.
+template <typename Real, int MAT, typename S4>
+__device__ __forceinline__ double psi_visit(const S4& uo, const S4& a, const S4& b, const S4& c,
+                                            int w, const RecTab<Real>& tab) {
+  if constexpr (sizeof(Real) == 8) {
+    const TetRows t = load_rows(tab, w);
+    double G[9];
+    slot_gradient64(uo, a, b, c, slot_place(w), t, G);
+    return psi_of<double, MAT>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], G[8], t.p0, t.p1);
+  } else {
+    const float4* t = tab.p + 3 * (size_t)w;
+    return double(slot_psi<Real, MAT>(Real(a.x - uo.x), Real(a.y - uo.y), Real(a.z - uo.z),
+                                      Real(b.x - uo.x), Real(b.y - uo.y), Real(b.z - uo.z),
+                                      Real(c.x - uo.x), Real(c.y - uo.y), Real(c.z - uo.z), t[0],
+                                      t[1], t[2]));
+  }
+}
+
 // Strain energies of the environment's tets (its tet list: one owner slot per
 // tet with a solved vertex, the slot's G taken relative to the owner, the
 // energy counted once at full weight), for the entries first, first + stride,
@@ -692,9 +968,8 @@ __device__ __forceinline__ Real slot_psi(Real d0x, Real d0y, Real d0z, Real d1x,
 // correction in the state precision).
 template <typename Real, typename SReal, int MAT, class State>
 __device__ __forceinline__ double2 tet_energy(const DevMesh& m, const EnvInfo& e,
-                                              const State& st, const real4<Real>* tab,
+                                              const State& st, const RecTab<Real>& tab,
                                               int first, int stride, bool pair) {
-  using R4 = real4<Real>;
   using S4 = real4<SReal>;
   auto shifted = [&](S4 v, int local_id) {
     const float4 d = m.ws_pred[e.vbase + local_id];
@@ -709,24 +984,14 @@ __device__ __forceinline__ double2 tet_energy(const DevMesh& m, const EnvInfo& e
   for (int i = first; i < e.ntets; i += stride) {
     const int4 id = __ldg(m.tet_slot + e.tbase + i);
     const int o = __ldg(m.tet_owner + e.tbase + i);
-    const R4* t = tab + 3 * (size_t)id.w;
-    const R4 q0 = t[0], q1 = t[1], q2 = t[2];
     const S4 uo = st.load(o);
     const S4 a = st.load(id.x);
     const S4 b = st.load(id.y);
     const S4 c = st.load(id.z);
-    acc += double(slot_psi<Real, MAT>(Real(a.x - uo.x), Real(a.y - uo.y), Real(a.z - uo.z),
-                                      Real(b.x - uo.x), Real(b.y - uo.y), Real(b.z - uo.z),
-                                      Real(c.x - uo.x), Real(c.y - uo.y), Real(c.z - uo.z), q0,
-                                      q1, q2));
-    if (pair) {
-      const S4 uob = shifted(uo, o);
-      const S4 ab = shifted(a, id.x), bb = shifted(b, id.y), cb = shifted(c, id.z);
-      accb += double(slot_psi<Real, MAT>(
-          Real(ab.x - uob.x), Real(ab.y - uob.y), Real(ab.z - uob.z), Real(bb.x - uob.x),
-          Real(bb.y - uob.y), Real(bb.z - uob.z), Real(cb.x - uob.x), Real(cb.y - uob.y),
-          Real(cb.z - uob.z), q0, q1, q2));
-    }
+    acc += psi_visit<Real, MAT>(uo, a, b, c, id.w, tab);
+    if (pair)
+      accb += psi_visit<Real, MAT>(shifted(uo, o), shifted(a, id.x), shifted(b, id.y),
+                                   shifted(c, id.z), id.w, tab);
   }
   return make_double2(acc, accb);
 }

@@ -159,10 +159,13 @@ int build_tet_data(const double* X, const int32_t* tets, int T, const double* rh
   return VBD_OK;
 }
 
-// Unique slot-record values (b_n0, p0, b_n1, p1, b_n2, p2).  Two slots share an
-// entry when their values are bitwise equal after conversion to the solver's
-// arithmetic precision, so sharing never changes a result.  Voxel meshes have
-// a handful of tet shapes, so thousands of slots map to one entry.
+// Unique record values, three rows of four.  fp32 arithmetic: one record per
+// distinct slot, (b_n0, p0, b_n1, p1, b_n2, energy weight).  fp64: one per
+// distinct tet, the rows of Dm^-1 (b_0, p0, b_1, p1, b_2, p0), shared by the
+// slots of its four vertices.  Two slots or tets share an entry when their
+// values are bitwise equal in the solver's arithmetic precision, so sharing
+// never changes a result.  Voxel meshes have a handful of tet shapes, so
+// thousands of slots map to one entry.
 struct RecordTable {
   bool fp64 = false;
   std::vector<double> vals;  // 12 per entry
@@ -396,6 +399,7 @@ int build_layout(const double* X, int V, const int32_t* tets, int T, const uint8
     L.rec_idx.resize((size_t)block_count * 32, make_int4(0, 0, 0, 0));
     RecordTable etab;
     etab.fp64 = L.table.fp64;
+    std::vector<int> tet_rec(etab.fp64 ? tn : 0, -1);  // fp64: record of each tet
     std::vector<std::pair<int, int4>> tlist;  // (owner, owner slot) per tet
     std::vector<int> old_of_new_local(vn);
     for (int v = 0; v < vn; ++v) old_of_new_local[new_local[v]] = v;
@@ -416,7 +420,6 @@ int build_layout(const double* X, int V, const int32_t* tets, int T, const uint8
             const int a = loc[off[ov] + j];
             const size_t blk = (size_t)ch.block + s;
             int ids[3];
-            double val[12];
             const double* bt = &td.b[(size_t)t * 12];
             const double* pt = &td.p[(size_t)t * 3];
             int n = 0, solved_in_tet = 0, owner = vn;
@@ -426,19 +429,34 @@ int build_layout(const double* X, int V, const int32_t* tets, int T, const uint8
                 ++solved_in_tet;
                 owner = std::min(owner, nl);
               }
-              if (qq == a) continue;
-              ids[n] = new_local[tets[4 * (size_t)t + qq] - vo];
-              val[4 * n + 0] = bt[qq * 3 + 0];
-              val[4 * n + 1] = bt[qq * 3 + 1];
-              val[4 * n + 2] = bt[qq * 3 + 2];
-              val[4 * n + 3] = pt[n];
-              ++n;
+              if (qq != a) ids[n++] = nl;
             }
-            // 4th value of the last plane: this slot's share of the tet's
-            // strain energy, so that summing over slots counts every tet with
-            // a solved vertex once (incremental-potential evaluation)
-            val[11] = 1.0 / solved_in_tet;
-            const int rid = etab.insert(val);
+            int rid;
+            if (etab.fp64) {
+              int& rec = tet_rec[t - to];
+              if (rec < 0) {
+                double val[12];
+                for (int i = 0; i < 3; ++i) {
+                  for (int c = 0; c < 3; ++c) val[4 * i + c] = bt[3 * i + c];
+                  val[4 * i + 3] = pt[i & 1];
+                }
+                rec = etab.insert(val);
+              }
+              rid = 4 * rec + a;
+            } else {
+              double val[12];
+              n = 0;
+              for (int qq = 0; qq < 4; ++qq) {
+                if (qq == a) continue;
+                for (int c = 0; c < 3; ++c) val[4 * n + c] = bt[qq * 3 + c];
+                val[4 * n + 3] = pt[n];
+                ++n;
+              }
+              // 4th value of the last row: this slot's share of the tet's
+              // strain energy
+              val[11] = 1.0 / solved_in_tet;
+              rid = etab.insert(val);
+            }
             L.rec_idx[blk * 32 + lane] = make_int4(ids[0], ids[1], ids[2], rid);
             if (owner == gv - vo) tlist.emplace_back(owner, make_int4(ids[0], ids[1], ids[2], rid));
             L.n_slots++;
@@ -1149,9 +1167,12 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     }
   }
   s->n_records = (long long)s->L.rec_idx.size();
-  // 16-bit slots when every environment-local id and record id fits
-  s->fmt = (s->L.max_env_vertices <= 65536 && s->L.max_env_records <= 65536) ? kFmtIdx16
-                                                                              : kFmtIdx32;
+  // 16-bit slots when every environment-local id and record id fits (an fp64
+  // slot's id holds its record and its vertex's place in the tet)
+  s->fmt = (s->L.max_env_vertices <= 65536 &&
+            s->L.max_env_records <= (s->fp64 ? 65536 / 4 : 65536))
+               ? kFmtIdx16
+               : kFmtIdx32;
 
   // ---- device upload --------------------------------------------------------
   auto bad = [&](cudaError_t e, const char* what) {

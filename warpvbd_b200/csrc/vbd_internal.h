@@ -19,12 +19,15 @@
 //              other three vertices and the environment-local id of its
 //              record (ushort4 or int4, RecordFormat below); padding slots
 //              are zero.
-//   records    per environment, the distinct (b_n0, p0) (b_n1, p1) (b_n2, w)
-//              Real4 triples of its slots (EnvInfo::rbase, nrec):
+//   records    three Real4 each, per environment (EnvInfo::rbase, nrec), with
 //              b_n = gradient of the tet's linear shape function of vertex n
 //              (a row of Dm^-1, or minus their sum), p0 = V*mu, p1 = V*lambda
-//              (material-adjusted), w = the slot's share of the tet's strain
-//              energy (1 / solved vertices of the tet).
+//              (material-adjusted):
+//              fp32 arithmetic: the distinct (b_n0, p0) (b_n1, p1) (b_n2, w) of
+//              its slots, w = the slot's share of the tet's strain energy (1 /
+//              solved vertices of the tet);
+//              fp64: the distinct (b_0, p0) (b_1, p1) (b_2, p0) of its tets; a
+//              slot's rid is then 4 x record + the vertex's place in the tet.
 #pragma once
 #include <cstdint>
 
@@ -85,10 +88,9 @@ struct LoopControl {
 };
 
 // Slot formats (both index the environment's table of distinct records, 3
-// Real4 each, so slots that share a tet shape, material and energy weight
-// share one entry):
+// Real4 each, which slots of equal values share):
 //   kFmtIdx32  int4    (n0, n1, n2, record id)                     16 B/slot
-//   kFmtIdx16  ushort4 (n0, n1, n2, record id), all values < 65536  8 B/slot
+//   kFmtIdx16  ushort4 (n0, n1, n2, record id), all values < 65536   8 B/slot
 enum RecordFormat : int { kFmtIdx32 = 1, kFmtIdx16 = 2 };
 
 struct DevMesh {

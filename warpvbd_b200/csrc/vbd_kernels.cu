@@ -95,7 +95,7 @@ __device__ __forceinline__ int env_sweeps(const DevMesh& m, const EnvInfo& e, co
                                           double tol, unsigned& stat, bool& converged,
                                           unsigned long long* s_red,
                                           unsigned long long (*s_conv)[kMaxGroup],
-                                          int* s_done, const real4<Real>* tab,
+                                          int* s_done, const RecTab<Real>& tab,
                                           unsigned long long* dxw, Real* s_split) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   constexpr int kPart = SplitBuf<TPV>::per_part;
@@ -170,7 +170,7 @@ __device__ __forceinline__ int env_sweeps(const DevMesh& m, const EnvInfo& e, co
 template <typename Real, typename SReal, int MAT, bool GROUP>
 __device__ double env_energy(const DevMesh& m, const EnvInfo& e, const SmemState<SReal>& st,
                              int rank, int g, const StepConst& sc, double* s_sum,
-                             double (*s_esum)[kMaxGroup], int buf, const real4<Real>* tab) {
+                             double (*s_esum)[kMaxGroup], int buf, const RecTab<Real>& tab) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int first = rank * blockDim.x + threadIdx.x, stride = g * blockDim.x;
   double acc = tet_energy<Real, SReal, MAT>(m, e, st, tab, first, stride, false).x;
@@ -209,7 +209,7 @@ __device__ double env_energy(const DevMesh& m, const EnvInfo& e, const SmemState
 template <typename Real, typename SReal, int MAT, bool GROUP>
 __device__ double2 env_energy_pair(const DevMesh& m, const EnvInfo& e, const SmemState<SReal>& st,
                                    int rank, int g, const StepConst& sc, double* s_sum,
-                                   double2* s_pair, const real4<Real>* tab) {
+                                   double2* s_pair, const RecTab<Real>& tab) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int first = rank * blockDim.x + threadIdx.x, stride = g * blockDim.x;
   const double2 el = tet_energy<Real, SReal, MAT>(m, e, st, tab, first, stride, true);
@@ -270,7 +270,7 @@ __device__ unsigned warm_start_stage(const DevMesh& m, const EnvInfo& e,
                                      const SmemState<SReal>& local, int rank, int g,
                                      const StepConst& sc, double* s_sum,
                                      double (*s_esum)[kMaxGroup], double2* s_pair,
-                                     const real4<Real>* tab) {
+                                     const RecTab<Real>& tab) {
   using S4 = real4<SReal>;
   const S4* UT = reinterpret_cast<const S4*>(m.ut) + e.vbase;
   auto place = [&](SReal alpha) {
@@ -331,14 +331,12 @@ __global__ void __launch_bounds__(512) env_step_kernel(DevMesh m, StepParams p,
   const StepConst sc = make_const(p);
   // the environment's record table: staged in shared memory after the state
   // when the launch reserved room for it (p.tab_in_smem), else read from
-  // global memory; either way a generic pointer to its 3 x nrec Real4
-  using R4 = real4<Real>;
-  const R4* gtab = reinterpret_cast<const R4*>(m.rec_tab) + 3 * (size_t)e.rbase;
-  const R4* tab = gtab;
+  // global memory
+  RecTab<Real> tab = global_table<Real>(m.rec_tab, e.rbase);
   if (p.tab_in_smem) {
-    R4* stab = reinterpret_cast<R4*>(smem_raw + tab_smem_offset<SReal>(e.nv));
-    for (int i = threadIdx.x; i < 3 * e.nrec; i += blockDim.x) stab[i] = ldg4(gtab + i);
-    tab = stab;  // visible to the block after the __syncthreads / cluster barrier below
+    unsigned char* stab = smem_raw + tab_smem_offset<SReal>(e.nv);
+    stage_table(stab, tab, e.nrec);
+    tab = staged(tab, stab);  // visible to the block after the barrier below
   }
   const double tol = tol_env ? tol_env[env] : p.tol;
   if (threadIdx.x == 0) s_stat = 0u;
@@ -450,8 +448,7 @@ __global__ void __launch_bounds__(256) color_kernel(DevMesh m, int color,
   unsigned long long* dxrec = ctl->iter + 1 == pp->max_iter ? m.dxmax : nullptr;
   if (q < ci.chunk_end)
     process_chunk<Real, SReal, TPV, MAT, FMT>(m, 0, ci, q, lane, state, sc, cmax, stat,
-                                              reinterpret_cast<const real4<Real>*>(m.rec_tab),
-                                              dxrec);
+                                              global_table<Real>(m.rec_tab, 0), dxrec);
   cmax = warp_max_u64(cmax);
   const unsigned st = __reduce_or_sync(0xffffffffu, stat);
   if (lane == 0) {
@@ -655,11 +652,10 @@ __global__ void __launch_bounds__(256) potential_kernel(DevMesh m, StepParams p,
                                                         const real4<SReal>* __restrict__ x,
                                                         double* __restrict__ out) {
   using S4 = real4<SReal>;
-  using R4 = real4<Real>;
   const EnvInfo e = m.env[blockIdx.x];
   const StepConst sc = make_const(p);
   const GlobalState<SReal> st{const_cast<S4*>(x) + e.vbase};  // read only
-  const R4* tab = reinterpret_cast<const R4*>(m.rec_tab) + 3 * (size_t)e.rbase;
+  const RecTab<Real> tab = global_table<Real>(m.rec_tab, e.rbase);
   double acc = tet_energy<Real, SReal, MAT>(m, e, st, tab, threadIdx.x, blockDim.x, false).x;
   const S4* U = reinterpret_cast<const S4*>(m.u) + e.vbase;
   const S4* V = reinterpret_cast<const S4*>(m.vel) + e.vbase;

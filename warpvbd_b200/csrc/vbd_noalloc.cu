@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256) noalloc_color_kernel(DevMesh m, int color
   unsigned long long* dxrec = ctl->iter + 1 == pp->max_iter ? m.dxmax : nullptr;
   if (q < ci.chunk_end)
     process_chunk<Real, SReal, TPV, MAT, FMT>(m, 0, ci, q, lane, state, sc, cmax, stat,
-                                              reinterpret_cast<const real4<Real>*>(m.rec_tab),
+                                              global_table<Real>(m.rec_tab, 0),
                                               dxrec);
   cmax = warp_max_u64(cmax);
   const unsigned st = __reduce_or_sync(0xffffffffu, stat);

@@ -209,13 +209,11 @@ __global__ void __launch_bounds__(512) persist_kernel(DevMesh m,
   // the mesh's record table: staged in this block's shared memory when the
   // launch reserved room for it (visible after the first barrier), else read
   // from global memory
-  using R4 = real4<Real>;
   extern __shared__ __align__(16) unsigned char psmem[];
-  const R4* tab = reinterpret_cast<const R4*>(m.rec_tab);
+  RecTab<Real> tab = global_table<Real>(m.rec_tab, 0);
   if (pp->tab_in_smem) {
-    R4* stab = reinterpret_cast<R4*>(psmem);
-    for (int i = threadIdx.x; i < 3 * e.nrec; i += blockDim.x) stab[i] = ldg4(tab + i);
-    tab = stab;
+    stage_table(psmem, tab, e.nrec);
+    tab = staged(tab, psmem);
   }
 
 #define VBD_GRID_SYNC()                                       \
