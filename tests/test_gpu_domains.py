@@ -1,0 +1,108 @@
+"""The persistent fp64 step by domains (vbd_domain.cu): every lanes-per-vertex variant and its
+edges -- one domain, partial chunks, vertices with more slots than a lane prefetches, fixed,
+free and massless parts -- against the FP64 oracle, and the path for meshes whose domains do
+not fit in shared memory against the per-colour graph mode."""
+import numpy as np
+import pytest
+
+from warpvbd_b200 import VBDSolver, _lib, scenes
+from oracle.oracle import OracleSolver
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(kw, steps=3, damping=0.0, material="snh", **opt):
+    kw = dict(kw, damping_coefficient=damping, dx_tol=1e-7, max_iter=1000)
+    sol = VBDSolver(**kw, mode="persist", material=material, allow_high_valence=True, **opt)
+    orc = OracleSolver(**kw, material=material, guarded=True)
+    X = kw["initial_positions"]
+    diag = float(np.linalg.norm(X.max(0) - X.min(0)))
+    for _ in range(steps):
+        x = sol.step(sol.old_positions, 1e-3).numpy()
+        y = orc.step(None, 1e-3)
+        assert sol.last_iterations == orc.last_iterations
+        assert np.abs(x - y).max() < 1e-10 * diag
+    return sol
+
+
+@pytest.mark.parametrize("tpv", [0, 2, 4, 8, 16])
+@pytest.mark.parametrize("shape,material,damping", [
+    ((2, 1, 1), "snh", 0.0),     # 8 solved vertices: one domain
+    ((5, 2, 1), "stvk", 0.0),    # 30: two domains
+    ((13, 3, 2), "snh", 1.0),    # ragged domains and chunks, the default damping
+    ((33, 4, 3), "stvk", 0.0),   # 660: 55 domains
+])
+def test_domains_match_oracle(shape, material, damping, tpv):
+    s = scenes.cantilever(*shape)
+    _check(s.solver_kwargs(), material=material, damping=damping, tpv=tpv,
+           block_threads=64 if tpv == 2 else 0)
+
+
+@pytest.mark.parametrize("tpv", [0, 4])
+def test_fan_of_many_tets_with_free_and_fixed_vertices(tpv):
+    """Two vertices shared by 47 tets (more slots than a lane prefetches), a vertex in no tet
+    and fixed vertices."""
+    n = 47
+    a = np.arange(n + 1) / (n + 1) * 2 * np.pi
+    ring = np.stack([np.cos(a), np.sin(a), 0 * a], 1)
+    X = np.concatenate([[[0, 0, 0.6], [0, 0, -0.6]], ring, [[3.0, 0, 0]]]) * 0.1
+    tets = np.array([[0, 2 + i, 3 + i, 1] for i in range(n)], np.int32)
+    active = np.ones(len(X), bool)
+    active[2:8] = False
+    T = len(tets)
+    _check(dict(initial_positions=X, elements=tets, densities=np.full(T, 1000.0),
+                youngs_modulus=np.full(T, 5e5), poissons_ratio=np.full(T, 0.4),
+                active_mask=active), tpv=tpv)
+
+
+def test_warm_start_rejected_prediction_is_plain():
+    """A network that predicts nonsense is rejected by the potential check: positions and
+    sweep counts are the plain step's, bit for bit."""
+    from warpvbd_b200 import warmstart
+    s = scenes.cantilever(24, 3, 3)
+    a = VBDSolver(**s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1000,
+                  mode="persist")
+    b = VBDSolver(**s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1000,
+                  mode="persist")
+    p = warmstart.init_params(3)
+    p[-3:] = 1e4
+    b.set_warmstart(p)
+    for _ in range(4):
+        x = a.step(a.old_positions, 1e-3).numpy()
+        y = b.step(b.old_positions, 1e-3).numpy()
+        assert a.last_iterations == b.last_iterations
+        assert np.array_equal(x, y)
+
+
+def test_expired_wait_reports_timeout_and_the_solver_recovers():
+    s = scenes.cantilever(40)
+    p = VBDSolver(**s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1000,
+                  mode="persist")
+    L = _lib.load()
+    assert L.vbd_set_wait_limits(p._h, 0, 0) == 0
+    with pytest.raises(_lib.VBDError) as ei:
+        for _ in range(3):
+            p.step(p.old_positions, 1e-3)
+    assert ei.value.status == _lib.ERR_TIMEOUT
+    assert L.vbd_set_wait_limits(p._h, 1 << 26, 2_000_000_000) == 0
+    p.reset()
+    q = VBDSolver(**s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1000,
+                  mode="persist")
+    for _ in range(3):
+        assert np.array_equal(p.step(p.old_positions, 1e-3).numpy(),
+                              q.step(q.old_positions, 1e-3).numpy())
+
+
+def test_meshes_whose_domains_do_not_fit_match_graph_mode():
+    """320,000 different tets: a domain's records alone exceed a block's shared memory."""
+    s = scenes.cantilever(160, 20, 20)
+    rng = np.random.default_rng(1)
+    s.vertices = s.vertices + rng.uniform(-0.08, 0.08, s.vertices.shape) * s.meta["voxel"]
+    kw = dict(s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-6, max_iter=1000)
+    p, g = VBDSolver(**kw, mode="persist"), VBDSolver(**kw, mode="graph")
+    diag = float(np.linalg.norm(s.vertices.max(0) - s.vertices.min(0)))
+    for _ in range(2):
+        x = p.step(p.old_positions, 1e-3).numpy()
+        y = g.step(g.old_positions, 1e-3).numpy()
+        assert p.last_iterations == g.last_iterations
+        assert np.abs(x - y).max() < 1e-13 * diag

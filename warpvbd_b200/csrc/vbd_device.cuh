@@ -308,7 +308,7 @@ __device__ __forceinline__ void slot_gradient64(const double4& uo, const double4
   G[8] = dot3(d0z, t.r0.z, d1z, t.r1.z, d2z, t.r2.z);
 }
 
-// 1 / x for x >= 1: the hardware's approximation and two Newton steps
+// 1 / x for normal x away from the ends of the range: the hardware's approximation and two Newton steps
 // y (2 - x y), each of which doubles its correct bits.
 __device__ __forceinline__ double reciprocal64(double x) {
   double y;
@@ -461,7 +461,7 @@ __device__ __forceinline__ bool solve3(const double* h, const double* g, double*
                c12 = cross2(h[1], h[2], h[0], h[4]), c22 = cross2(h[0], h[3], h[1], h[1]);
   const double det = dot3(h[0], c00, h[1], c01, h[2], c02);
   if (!(fabs(det) > 1e-250 && fabs(det) < 1e250)) return chol_solve3<double>(h, g, x);
-  const double r = -1.0 / det;
+  const double r = -reciprocal64(det);
   x[0] = dot3(c00, g[0], c01, g[1], c02, g[2]) * r;
   x[1] = dot3(c01, g[0], c11, g[1], c12, g[2]) * r;
   x[2] = dot3(c02, g[0], c12, g[1], c22, g[2]) * r;

@@ -12,17 +12,20 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
 #include "../../include/vbd_b200.h"
 #include "vbd_internal.h"
 #include "vbd_launch.h"
+#include "vbd_domain.h"
 #include "vbd_persist.h"
 #include "vbd_noalloc.h"
 #include "vbd_setup.h"
@@ -532,6 +535,23 @@ struct vbd_solver {
   DevBuf<int> d_nbr_off, d_nbr_idx;
   DevBuf<unsigned long long> d_epoch;
   bool persist_scoped = false;
+  // fp64 by domains (vbd_domain.cu): layouts of 1, `cluster` and `cluster_wide`
+  // domains per environment (block mode), or one of ndom (persistent mode)
+  bool by_domains = false;
+  int ndom = 0, dom_tpv = 0;
+  unsigned dom_seq = 0;
+  std::vector<size_t> dom_smem[3];  // per environment
+  DevBuf<int> d_dom_first[3];
+  DevBuf<DomInfo> d_dom;
+  DevBuf<DomColor> d_dom_color;
+  DevBuf<DomChunk> d_dom_chunk;
+  DevBuf<ushort4> d_dom_slot;
+  DevBuf<int2> d_dom_local;
+  DevBuf<double> d_dom_rec;
+  DevBuf<int4> d_dom_tet;
+  DevBuf<int> d_dom_tet_owner;
+  DevBuf<ulonglong2> d_dom_mail, d_dom_post;
+  DevBuf<unsigned> d_dom_abort;
   PersistLimits wait_limits{1ll << 26, 2000000000ull};  // every grid-barrier wait
   // block-mode work map: (environment, rank, group size) per thread block
   int cluster = 1;           // blocks per cluster = group size of a split environment
@@ -707,6 +727,18 @@ void free_solver(vbd_solver* s) {
   s->d_nbr_off.release();
   s->d_nbr_idx.release();
   s->d_epoch.release();
+  for (auto& f : s->d_dom_first) f.release();
+  s->d_dom_abort.release();
+  s->d_dom.release();
+  s->d_dom_color.release();
+  s->d_dom_chunk.release();
+  s->d_dom_slot.release();
+  s->d_dom_local.release();
+  s->d_dom_rec.release();
+  s->d_dom_tet.release();
+  s->d_dom_tet_owner.release();
+  s->d_dom_mail.release();
+  s->d_dom_post.release();
   if (s->h_iters) cudaFreeHost(s->h_iters);
   if (s->h_status) cudaFreeHost(s->h_status);
   if (s->h_dxmax) cudaFreeHost(s->h_dxmax);
@@ -758,8 +790,11 @@ size_t env_smem(const vbd_solver* s, const EnvInfo& ei, bool with_tab) {
 //   mixed precision, 4 lanes per vertex: A1 = 8300, I_C = 10300 / 11200 /
 //     12200 / 16500 (1.72 ns per slot visit; the 68K-slot environment 129 /
 //     78 / 49 / 35 / 36 us per sweep on 1 / 2 / 4 / 8 / 16 blocks)
-//   fp64, 2 lanes per vertex: A1 = 10200, I_C = 12900 / 13500 / 13900 / 18000
-//     (2.34 ns per slot visit; 183 / 112 / 67 / 54 / 55 us)
+//   fp64 by domains, 4 lanes per vertex: A1 = 7200, I_C = 9200 / 9700 / 10200 /
+//     11400 (2.15 ns per slot visit; 55K slots 133 / 84 / 54 / 36.6 / 30.5 us, 27K
+//     79 / 50 / 36 / 29 / 26 us, 7K 31 / 28 / 25 / 24 / 25 us)
+//   fp64 otherwise, 2 lanes per vertex: A1 = 10200, I_C = 12900 / 13500 / 13900 /
+//     18000 (2.34 ns per slot visit; 183 / 112 / 67 / 54 / 55 us)
 // (the fixed part is the per-colour barrier and dependency chain; at 16
 // blocks every store also goes to 15 replicas, which I_16 absorbs).  With cluster > 1 the longest environments may each take a whole
 // cluster (group = cluster); the split set is the one with the smallest
@@ -773,11 +808,12 @@ size_t env_smem(const vbd_solver* s, const EnvInfo& ei, bool with_tab) {
 // then starts first.
 // I_C of the duration model: measured at C = 2, 4, 8, 16, linear in C between
 // those points (C = 3, 5-7, 9-15).
-double split_overhead(int C, bool fp64) {
+double split_overhead(int C, bool fp64, bool by_domains) {
   static const double c[4] = {2.0, 4.0, 8.0, 16.0};
   static const double vm[4] = {10300.0, 11200.0, 12200.0, 16500.0};
   static const double vd[4] = {12900.0, 13500.0, 13900.0, 18000.0};
-  const double* v = fp64 ? vd : vm;
+  static const double vs[4] = {9200.0, 9700.0, 10200.0, 11400.0};
+  const double* v = by_domains ? vs : (fp64 ? vd : vm);
   if (C <= 2) return v[0];
   for (int i = 1; i < 4; ++i)
     if (C <= c[i]) return v[i - 1] + (v[i] - v[i - 1]) * (C - c[i - 1]) / (c[i] - c[i - 1]);
@@ -800,9 +836,9 @@ void make_plan(const vbd_solver* s, const int* iters, std::vector<int4>& work,
   work2.clear();
   work3.clear();
   const bool f64 = s->prec == 2;
-  const double a1 = f64 ? 10200.0 : 8300.0;
-  const double aC = split_overhead(C, f64);
-  const double aW = Cw > 1 ? split_overhead(Cw, f64) : 0.0;
+  const double a1 = s->by_domains ? 7200.0 : (f64 ? 10200.0 : 8300.0);
+  const double aC = split_overhead(C, f64, s->by_domains);
+  const double aW = Cw > 1 ? split_overhead(Cw, f64, s->by_domains) : 0.0;
   // high and mean estimates on one block, on C blocks and on Cw blocks
   std::vector<double> d1(n), dC(n), dW(n), m1(n), mC(n), mW(n);
   const bool hist = s->env_sweeps.size() == (size_t)n && s->env_sweeps_mean.size() == (size_t)n &&
@@ -910,7 +946,10 @@ void make_plan(const vbd_solver* s, const int* iters, std::vector<int4>& work,
 size_t tier_smem(const vbd_solver* s, const std::vector<int4>& w) {
   size_t need = 0;
   for (const int4& x : w)
-    if (x.x >= 0) need = std::max(need, env_smem(s, s->L.env[x.x], s->tab_in_smem));
+    if (x.x >= 0)
+      need = std::max(need, s->by_domains
+                                ? s->dom_smem[x.z == 1 ? 0 : (x.z == s->cluster ? 1 : 2)][x.x]
+                                : env_smem(s, s->L.env[x.x], s->tab_in_smem));
   return need;
 }
 
@@ -1002,6 +1041,320 @@ void build_persist_neighbours(const Layout& L, int tpv, int nwarps, int nb, std:
   }
 }
 
+// ---------------------------------------------------------------------------
+// Domains of the fp64 step (vbd_domain.cu): an environment's solved vertices
+// divided by recursive bisection of their rest positions (along the longest
+// side, by incident tets), and for each domain its vertices, slots, records and
+// tets in local ids.
+// ---------------------------------------------------------------------------
+struct DomLayout {
+  std::vector<DomInfo> dom;
+  std::vector<DomColor> color;
+  std::vector<DomChunk> chunk;
+  std::vector<ushort4> slot;
+  std::vector<int2> local;
+  std::vector<double> rec;
+  std::vector<int4> tet_slot;
+  std::vector<int> tet_owner;
+  bool fits = true;  // positions in a block's shared memory, ids in 16 bits
+
+  // Appends another layout, its offsets moved behind this one's.
+  void append(const DomLayout& o) {
+    const int nd = (int)dom.size(), nc = (int)color.size(), nq = (int)chunk.size();
+    const int nb = (int)(slot.size() / 32), nl = (int)local.size(), nr = (int)(rec.size() / 12);
+    const int nt = (int)tet_slot.size();
+    fits = fits && o.fits;
+    dom.insert(dom.end(), o.dom.begin(), o.dom.end());
+    for (size_t i = nd; i < dom.size(); ++i) {
+      dom[i].lbase += nl;
+      dom[i].rbase += nr;
+      dom[i].tbase += nt;
+      dom[i].qbase += nq;
+      dom[i].cbase += nc;
+    }
+    chunk.insert(chunk.end(), o.chunk.begin(), o.chunk.end());
+    for (size_t i = nq; i < chunk.size(); ++i) chunk[i].block += nb;
+    color.insert(color.end(), o.color.begin(), o.color.end());
+    slot.insert(slot.end(), o.slot.begin(), o.slot.end());
+    local.insert(local.end(), o.local.begin(), o.local.end());
+    rec.insert(rec.end(), o.rec.begin(), o.rec.end());
+    tet_slot.insert(tet_slot.end(), o.tet_slot.begin(), o.tet_slot.end());
+    tet_owner.insert(tet_owner.end(), o.tet_owner.begin(), o.tet_owner.end());
+  }
+};
+
+void bisect(const std::vector<double>& x, const int* weight, std::vector<int>& ids, size_t begin,
+            size_t end, int first, int parts, std::vector<int>& owner) {
+  if (parts == 1) {
+    for (size_t i = begin; i < end; ++i) owner[ids[i]] = first;
+    return;
+  }
+  double lo[3], hi[3];
+  for (int c = 0; c < 3; ++c) {
+    lo[c] = 1e300;
+    hi[c] = -1e300;
+  }
+  long long total = 0;
+  for (size_t i = begin; i < end; ++i) {
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = std::min(lo[c], x[3 * (size_t)ids[i] + c]);
+      hi[c] = std::max(hi[c], x[3 * (size_t)ids[i] + c]);
+    }
+    total += weight[ids[i]];
+  }
+  int axis = 0;
+  for (int c = 1; c < 3; ++c)
+    if (hi[c] - lo[c] > hi[axis] - lo[axis]) axis = c;
+  std::vector<std::pair<double, int>> key(end - begin);
+  for (size_t i = begin; i < end; ++i) key[i - begin] = {x[3 * (size_t)ids[i] + axis], ids[i]};
+  std::sort(key.begin(), key.end());
+  const int left = parts / 2;
+  const long long want = total * left / parts;
+  long long sum = 0;
+  size_t mid = begin;
+  for (size_t i = begin; i < end; ++i) {
+    ids[i] = key[i - begin].second;
+    if (sum < want) mid = i + 1;
+    sum += weight[ids[i]];
+  }
+  // every part keeps a vertex while there are enough
+  if (end - begin >= (size_t)parts)
+    mid = std::min(std::max(mid, begin + left), end - (parts - left));
+  bisect(x, weight, ids, begin, mid, first, left, owner);
+  bisect(x, weight, ids, mid, end, first + left, parts - left, owner);
+}
+
+// Blocks a single mesh of ns solved vertices is divided among: one per SM, down
+// to a dozen vertices a block.  fp64 us per sweep on B200 with 6 / 12 / 24 vertices
+// a domain: 20x2x2 beam 13.7 / 13.7 / 14.9, 40x4x4 beam 14.7 / 15.2 / 17.0, 11^3
+// mass-spring (148 / 148 / 75 domains) 19.1 / 19.1 / 18.5; the 80x8x8 beam on 148 /
+// 67 domains 18.9 / 25.6.
+int domain_count(int ns, int sms) {
+  return std::min(std::min(sms, kDomMaxBlocks), std::max(1, ns / 12));
+}
+
+// Lanes per vertex for domains of n vertices.  Few vertices: a colour's time is
+// one vertex's chain of slots, so more lanes (32 against 16 at 12 vertices 15.2 /
+// 16.3 us per sweep, 16 against 8 at 44: 18.9 / 19.2).  Many: the fp64 pipe is
+// the limit and every lane beyond four adds idle ones (4 against 8 at 312
+// vertices 33.1 / 34.5, at 2,350: 116 / 154; 2 lanes 137).
+int domain_tpv(int n) { return n <= 16 ? 32 : (n <= 64 ? 16 : (n <= 160 ? 8 : 4)); }
+
+// Environment k in ndom domains.  X: rest positions, caller order; ltpv, tpv:
+// lanes per vertex of the solver's layout and of the domains'.
+void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, int ndom,
+                   bool sort_records, DomLayout& D) {
+  const EnvInfo& e = L.env[k];
+  const int V = e.nv, ns = e.nsolved, C = e.ncolors, cpw = 32 / tpv, lcpw = 32 / ltpv;
+  const int* valence = L.valence.data() + e.vbase;
+  std::vector<double> x(3 * (size_t)V);
+  for (int v = 0; v < V; ++v)
+    for (int c = 0; c < 3; ++c)
+      x[3 * (size_t)(L.new_of_old[e.vbase + v] - e.vbase) + c] = X[3 * (size_t)(e.vbase + v) + c];
+  std::vector<int> owner(V, -1), ids(ns), color(ns);
+  for (int i = 0; i < ns; ++i) ids[i] = i;
+  bisect(x, valence, ids, 0, ns, 0, ndom, owner);
+  for (int c = 0; c < C; ++c)
+    for (int v = L.color[e.cbase + c].vbegin; v < L.color[e.cbase + c].vend; ++v)
+      color[v - e.vbase] = c;
+  // the slots of vertex v in the solver's layout
+  auto slot_of = [&](int v, int j) -> const int4& {
+    const ColorInfo& ci = L.color[e.cbase + color[v]];
+    const int p = e.vbase + v - ci.vbegin;
+    const ChunkInfo& ch = L.chunk[ci.chunk_begin + p / lcpw];
+    return L.rec_idx[((size_t)ch.block + j / ltpv) * 32 + p % lcpw * ltpv + j % ltpv];
+  };
+  std::vector<std::vector<int>> own(ndom);
+  for (int v = 0; v < ns; ++v) own[owner[v]].push_back(v);  // by colour, as numbered
+  // inside a colour: by valence, then by the records of its slots, so that the
+  // vertices of a chunk read the same records at the same time where they can
+  // (67 instead of 84 shared-memory wavefronts per 32 slots on the 160x16x16 beam,
+  // with the lane order of DomChunk)
+  if (sort_records)
+    for (auto& o : own)
+      std::sort(o.begin(), o.end(), [&](int a, int b) {
+        if (color[a] != color[b]) return color[a] < color[b];
+        if (valence[a] != valence[b]) return valence[a] > valence[b];
+        for (int j = 0; j < valence[a]; ++j) {
+          const int ra = slot_of(a, j).w, rb = slot_of(b, j).w;
+          if (ra != rb) return ra < rb;
+        }
+        return a < b;
+      });
+  std::vector<std::vector<int>> tets(ndom);
+  for (int t = e.tbase; t < e.tbase + e.ntets; ++t) tets[owner[L.tet_owner[t]]].push_back(t);
+  std::vector<char> mailed(ns, 0);
+  std::vector<int> loc(V, -1), rec_loc(e.nrec, -1), others, recs;
+  for (int r = 0; r < ndom; ++r) {
+    DomInfo di{};
+    di.env = k;
+    di.nd = ndom;
+    di.rank = r;
+    di.lbase = (int)D.local.size();
+    di.nown = (int)own[r].size();
+    di.rbase = (int)(D.rec.size() / 12);
+    di.tbase = (int)D.tet_slot.size();
+    di.qbase = (int)D.chunk.size();
+    di.cbase = (int)D.color.size();
+    di.ncolors = C;
+    for (int i = 0; i < di.nown; ++i) loc[own[r][i]] = i;
+    // the other vertices of its tets: solved ones by colour, then the unsolved
+    others.clear();
+    for (int v : own[r])
+      for (int j = 0; j < valence[v]; ++j) {
+        const int4& s = slot_of(v, j);
+        for (int n : {s.x, s.y, s.z})
+          if (loc[n] < 0) {
+            loc[n] = 0;
+            others.push_back(n);
+          }
+      }
+    std::sort(others.begin(), others.end());
+    for (size_t i = 0; i < others.size(); ++i) loc[others[i]] = di.nown + (int)i;
+    di.nloc = di.nown + (int)others.size();
+    for (int v : own[r]) D.local.push_back(make_int2(e.vbase + v, valence[v]));
+    for (int n : others) {
+      D.local.push_back(make_int2(e.vbase + n, 0));
+      if (n < ns) mailed[n] = 1;
+    }
+    recs.clear();
+    auto local_slot = [&](const int4& s) {
+      int& q = rec_loc[s.w >> 2];
+      if (q < 0) {
+        q = (int)recs.size();
+        recs.push_back(s.w >> 2);
+      }
+      return make_int4(loc[s.x], loc[s.y], loc[s.z], 4 * q + (s.w & 3));
+    };
+    size_t h = 0;
+    int at = 0;
+    for (int c = 0; c < C; ++c) {
+      DomColor dc{};
+      dc.chunk_begin = (int)D.chunk.size() - di.qbase;
+      int end = at;
+      while (end < di.nown && color[own[r][end]] == c) ++end;
+      for (; at < end; at += cpw) {
+        const int n = std::min(cpw, end - at);
+        int kmax = 0;
+        for (int i = 0; i < n; ++i) kmax = std::max(kmax, valence[own[r][at + i]]);
+        DomChunk ch{(int)(D.slot.size() / 32), (kmax + tpv - 1) / tpv, at, at + n};
+        D.slot.resize(D.slot.size() + 32 * (size_t)ch.steps, make_ushort4(0, 0, 0, 0));
+        for (int i = 0; i < n; ++i)
+          for (int j = 0; j < valence[own[r][at + i]]; ++j) {
+            const int4 s = local_slot(slot_of(own[r][at + i], j));
+            D.slot[((size_t)ch.block + j / tpv) * 32 + j % tpv * cpw + i] =
+                make_ushort4((unsigned short)s.x, (unsigned short)s.y, (unsigned short)s.z,
+                             (unsigned short)s.w);
+          }
+        D.chunk.push_back(ch);
+      }
+      at = end;
+      dc.chunk_end = (int)D.chunk.size() - di.qbase;
+      dc.halo_begin = di.nown + (int)h;
+      while (h < others.size() && others[h] < ns && color[others[h]] == c) ++h;
+      dc.halo_end = di.nown + (int)h;
+      D.color.push_back(dc);
+    }
+    di.nchunk = (int)D.chunk.size() - di.qbase;
+    for (int t : tets[r]) {
+      D.tet_owner.push_back(loc[L.tet_owner[t]]);
+      D.tet_slot.push_back(local_slot(L.tet_slot[t]));
+    }
+    di.ntets = (int)tets[r].size();
+    di.nrec = (int)recs.size();
+    for (int q : recs) {
+      const double* v = &L.table.vals[12 * (size_t)(e.rbase + q)];
+      D.rec.insert(D.rec.end(), v, v + 12);
+    }
+    // shared memory: the records first, then the chunk and vertex lists
+    for (int f : {kDomRecords, kDomMeta})
+      if (dom_smem(di.nloc, di.nrec, di.nchunk, di.flags | f) <= kDomMaxSmem) di.flags |= f;
+    D.fits = D.fits && dom_smem(di.nloc, 0, 0, 0) <= kDomMaxSmem && di.nloc <= 65536 &&
+             di.nrec <= 65536 / 4 && C <= kDomMaxColors;
+    D.dom.push_back(di);
+    for (int v : own[r]) loc[v] = -1;
+    for (int n : others) loc[n] = -1;
+    for (int q : recs) rec_loc[q] = -1;
+    if (!D.fits) return;
+  }
+  for (const DomInfo& di : D.dom)
+    for (int l = di.lbase; l < di.lbase + di.nown; ++l)
+      if (mailed[D.local[l].x - e.vbase]) D.local[l].x = ~D.local[l].x;
+}
+
+// Every environment in `parts` domains, appended to D; first[env] = its first
+// domain, smem[env] = the largest of its domains'.  The environments are
+// independent: host threads take them in turn.
+void build_all_domains(const Layout& L, int ltpv, const double* X, int tpv, int parts,
+                       bool sort_records, DomLayout& D, std::vector<int>& first,
+                       std::vector<size_t>& smem) {
+  const int n = (int)L.env.size();
+  std::vector<DomLayout> each(n);
+  std::atomic<int> next{0};
+  auto work = [&]() {
+    for (int k; (k = next.fetch_add(1)) < n;)
+      build_domains(L, ltpv, X, k, tpv, parts, sort_records, each[k]);
+  };
+  const int nthreads =
+      std::min<int>(n, std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
+  std::vector<std::thread> pool;
+  for (int i = 1; i < nthreads; ++i) pool.emplace_back(work);
+  work();
+  for (auto& t : pool) t.join();
+  first.resize(n);
+  smem.assign(n, 0);
+  for (int k = 0; k < n; ++k) {
+    first[k] = (int)D.dom.size();
+    for (const DomInfo& di : each[k].dom)
+      smem[k] = std::max(smem[k], dom_smem(di.nloc, di.nrec, di.nchunk, di.flags));
+    D.append(each[k]);
+    each[k] = DomLayout();
+  }
+}
+
+// The next step's number (vbd_domain.h: tags), and the arrays of a launch.
+DomDev dom_dev(const vbd_solver* s) {
+  DomDev d{};
+  d.dom = s->d_dom.p;
+  d.color = s->d_dom_color.p;
+  d.chunk = s->d_dom_chunk.p;
+  d.slot = s->d_dom_slot.p;
+  d.local = s->d_dom_local.p;
+  d.rec = reinterpret_cast<const double4*>(s->d_dom_rec.p);
+  d.tet_slot = s->d_dom_tet.p;
+  d.tet_owner = s->d_dom_tet_owner.p;
+  d.mail = s->d_dom_mail.p;
+  d.post = s->d_dom_post.p;
+  d.abort = s->d_dom_abort.p;
+  d.seq = s->dom_seq;
+  d.grid_sync = (s->flags & VBD_PERSIST_GRID_BARRIERS) ? 1 : 0;
+  return d;
+}
+
+// Resident blocks per SM (cluster = 1) or resident clusters of the block mode's
+// kernel at the solver's largest shared memory.
+cudaError_t block_occupancy(const vbd_solver* s, int threads, int cluster, int* out) {
+  return s->by_domains
+             ? dom_occupancy(s->material, s->dom_tpv, threads, s->smem_bytes, cluster, out)
+             : env_occupancy(s->prec, s->material, s->fmt, s->tpv, threads, s->smem_bytes, cluster,
+                             out);
+}
+
+// One block-mode launch over a work map.
+cudaError_t launch_block(const vbd_solver* s, const DevMesh& m, const StepParams& p,
+                         const double* tol, const int4* work, int n_blocks, int cluster,
+                         int threads, size_t smem, cudaStream_t st) {
+  if (!s->by_domains)
+    return launch_env_step(s->prec, s->material, s->tpv, threads, m, p, tol, work, n_blocks,
+                           cluster, smem, st);
+  DomDev d = dom_dev(s);
+  d.work = work;
+  d.first_single = s->d_dom_first[0].p;
+  d.first_split = s->d_dom_first[cluster == s->cluster ? 1 : 2].p;
+  return launch_domain(s->material, s->dom_tpv, threads, m, p, d, tol, s->wait_limits, n_blocks,
+                       cluster, false, smem, st);
+}
+
 int create_impl(const double* X, int V, const int32_t* tets, int T, const double* rho,
                 const double* E, const double* nu, const uint8_t* active, double kd,
                 const double* gravity, const int32_t* coloring, const std::vector<int>& voff,
@@ -1059,6 +1412,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     }
   }
   // mode / threads / tpv
+  const bool tpv_given = tpv != 0, threads_given = threads != 0;
   int mode = flags & VBD_MODE_MASK;
   // provisional environment size bound for the shared-memory check
   int max_env_v = 0;
@@ -1068,13 +1422,16 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   const size_t smem_need = (size_t)max_env_v * smem_per_vertex;
   const bool fits = smem_need <= (size_t)env_kernel_max_smem();
   if (mode == VBD_MODE_AUTO) {
-    // measured on B200 (the autotuner's results for cantilever meshes):
-    // one block, or one cluster, holding the mesh in shared memory wins up
-    // to ~2k vertices; beyond that the persistent kernel over the whole GPU
+    // measured on B200 (the autotuner's results for cantilever meshes): one block,
+    // or one cluster, holding the mesh in shared memory wins up to ~2k vertices;
+    // beyond that the persistent kernel over the whole GPU.  In fp64 the
+    // persistent step by domains wins from a few dozen vertices on (us per sweep,
+    // one block or cluster -> domains: 189 vertices 18.9 -> 13.7, 1,025 vertices
+    // 41 -> 15, 1,808 vertices 44 -> 19).
     if (s->n_env > 1)
       mode = VBD_MODE_BLOCK;
     else
-      mode = (fits && V <= 2048) ? VBD_MODE_BLOCK : VBD_MODE_PERSIST;
+      mode = (fits && V <= (s->fp64 ? 96 : 2048)) ? VBD_MODE_BLOCK : VBD_MODE_PERSIST;
   }
   if (mode == VBD_MODE_BLOCK && !fits) {
     delete s;
@@ -1099,7 +1456,12 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     delete s;
     return fail(VBD_ERR_INVALID_ARG, "cluster size must be 0 (automatic) or 1 to 16");
   }
-  s->cluster = !block_mode ? 1 : (cl ? cl : (s->n_env > 1 ? 4 : (V > 512 ? 8 : 1)));
+  // fp64: as many blocks per environment as there are SMs to go round (kernel ms
+  // of three steps with clusters of 16 / 8 / 4: 6 uneven environments 5.0 / 6.1 /
+  // 9.0, 16 environments 8.5 / 8.7 / 9.5, 40 environments - / 10.1 / 10.8)
+  const int cl_auto = s->n_env > 1 ? (s->fp64 ? (s->n_env <= 9 ? 16 : (s->n_env <= 48 ? 8 : 4)) : 4)
+                                   : (V > 512 ? 8 : 1);
+  s->cluster = !block_mode ? 1 : (cl ? cl : cl_auto);
   s->replan = block_mode && s->n_env > 1 && s->cluster > 1;
   s->tiered = s->replan && (flags & VBD_TIERED) != 0;
   // the wide tier: clusters twice the size of the split environments' (at
@@ -1108,7 +1470,8 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
                         ? std::min(16, 2 * s->cluster)
                         : 0;
   if (threads == 0)
-    threads = block_mode ? (s->n_env > 1 ? 256 : 512) : (mode == VBD_MODE_PERSIST ? 128 : 256);
+    threads = block_mode ? (s->n_env > 1 && !s->fp64 ? 256 : 512)
+                         : (mode == VBD_MODE_PERSIST ? 128 : 256);
   if (mode == VBD_MODE_GRAPH || mode == VBD_MODE_HOSTLOOP) threads = 256;
   if (threads % 32 || threads < 32 || threads > 512) {
     delete s;
@@ -1246,8 +1609,80 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   if (!err && bad(s->d_dxmax.alloc(s->n_env), "dxmax")) err = 1;
   if (!err && bad(s->d_params.alloc(1), "params")) err = 1;
   if (!err && bad(s->d_ctl.alloc(1), "ctl")) err = 1;
-  if (!err && mode == VBD_MODE_PERSIST) {
-    if (bad(s->d_pctl.alloc(1), "persist ctl")) err = 1;
+  if (!err && mode == VBD_MODE_PERSIST && bad(s->d_pctl.alloc(1), "persist ctl")) err = 1;
+  if (!err && s->fp64 && (block_mode || mode == VBD_MODE_PERSIST)) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const bool sort_records = (flags & VBD_ORDER_INDEX) == 0;
+    // layouts: persistent mode one; block mode 1, cluster and cluster_wide domains
+    // (a single environment in a cluster is never on one block)
+    int parts[3] = {0, 0, 0};
+    if (!block_mode) {
+      parts[0] = domain_count(s->L.env[0].nsolved, sms);
+    } else {
+      parts[0] = s->n_env > 1 || s->cluster == 1 ? 1 : 0;
+      parts[1] = s->cluster > 1 ? s->cluster : 0;
+      parts[2] = s->cluster_wide;
+    }
+    long long solved = 0;
+    for (const EnvInfo& ei : s->L.env) solved += ei.nsolved;
+    const int per = (int)(solved / s->n_env / std::max(1, s->n_env > 1 ? 1 : parts[0] + parts[1]));
+    // a batch's single blocks have registers for four lanes per vertex and more
+    // (with two, ten slots of a lane are held ahead: 83 instead of 79 us per
+    // sweep of 27K slots)
+    s->dom_tpv = tpv_given ? (s->n_env > 1 ? std::max(4, s->tpv) : s->tpv)
+                           : (s->n_env > 1 ? 4 : domain_tpv(per));
+    if (!block_mode && !threads_given) s->threads = per <= 64 ? 256 : 512;
+    DomLayout D;
+    std::vector<int> first[3];
+    for (int i = 0; i < 3 && D.fits; ++i)
+      if (parts[i] > 0)
+        build_all_domains(s->L, s->tpv, X, s->dom_tpv, parts[i], sort_records, D, first[i],
+                          s->dom_smem[i]);
+    int resident = 0;
+    if (D.fits && !block_mode) {
+      if (bad(dom_occupancy(s->material, s->dom_tpv, s->threads, s->dom_smem[0][0], 1, &resident),
+              "persist occupancy"))
+        err = 1;
+    }
+    if (!err && D.fits && (block_mode || resident * sms >= parts[0])) {
+      s->by_domains = true;
+      if (!block_mode) s->persist_blocks = s->ndom = parts[0];
+      int posts = 0;
+      bool split = false;
+      for (DomInfo& di : D.dom) {
+        if (di.rank == 0) posts += 2 * di.nd;
+        di.pbase = posts - 2 * di.nd;
+        split = split || di.nd > 1;
+      }
+      for (int i = 0; i < 3 && !err; ++i)
+        if (parts[i] > 0 && bad(s->d_dom_first[i].upload(first[i], st), "domains")) err = 1;
+      if (err || bad(s->d_dom.upload(D.dom, st), "domains") ||
+          bad(s->d_dom_color.upload(D.color, st), "domains") ||
+          bad(s->d_dom_chunk.upload(D.chunk, st), "domains") ||
+          bad(s->d_dom_slot.upload(D.slot, st), "domains") ||
+          bad(s->d_dom_local.upload(D.local, st), "domains") ||
+          bad(s->d_dom_rec.upload(D.rec, st), "domains") ||
+          bad(s->d_dom_tet.upload(D.tet_slot, st), "domains") ||
+          bad(s->d_dom_tet_owner.upload(D.tet_owner, st), "domains") ||
+          bad(s->d_dom_mail.alloc(split ? 3 * (size_t)V : 1), "domains") ||
+          bad(s->d_dom_post.alloc((size_t)posts), "domains") ||
+          bad(s->d_dom_abort.alloc(1), "domains") ||
+          bad(cudaMemsetAsync(s->d_dom_mail.p, 0, sizeof(ulonglong2) * s->d_dom_mail.n, st),
+              "domains") ||
+          bad(cudaMemsetAsync(s->d_dom_post.p, 0, sizeof(ulonglong2) * s->d_dom_post.n, st),
+              "domains") ||
+          bad(cudaMemsetAsync(s->d_dom_abort.p, 0, sizeof(unsigned), st), "domains"))
+        err = 1;
+      cudaStreamSynchronize(st);  // D and first go out of scope
+      if (block_mode) {
+        s->smem_bytes = 0;
+        for (const auto& v : s->dom_smem)
+          for (size_t x : v) s->smem_bytes = std::max(s->smem_bytes, x);
+      }
+    }
+  }
+  if (!err && mode == VBD_MODE_PERSIST && !s->by_domains) {
     // resident blocks, but no more than the largest colour can keep busy
     // (one chunk per warp): fewer blocks make cheaper grid barriers
     int per_sm = 0, sms = 0;
@@ -1335,20 +1770,14 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     if (s->tiered) {
       // capacity of the light launch (one block per environment) at the
       // largest environment's shared memory: a lower bound
-      if (bad(env_occupancy(s->prec, s->material, s->fmt, s->tpv, s->threads, s->smem_bytes, 1,
-                            &occ),
-              "occupancy"))
+      if (bad(block_occupancy(s, s->threads, 1, &occ), "occupancy"))
         err = 1;
       s->capacity_blocks = occ * sms;
       int occ_c = 0, occ_w = 0;
-      if (!err && bad(env_occupancy(s->prec, s->material, s->fmt, s->tpv, s->heavy_threads,
-                                    s->smem_bytes, s->cluster, &occ_c),
-                      "occupancy"))
+      if (!err && bad(block_occupancy(s, s->heavy_threads, s->cluster, &occ_c), "occupancy"))
         err = 1;
       if (!err && s->cluster_wide > 0 &&
-          bad(env_occupancy(s->prec, s->material, s->fmt, s->tpv, s->heavy_threads,
-                            s->smem_bytes, s->cluster_wide, &occ_w),
-              "occupancy"))
+          bad(block_occupancy(s, s->heavy_threads, s->cluster_wide, &occ_w), "occupancy"))
         err = 1;
       s->max_clusters_split = occ_c;
       s->max_clusters_wide = occ_w;
@@ -1363,9 +1792,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
            bad(s->d_work3.alloc((size_t)s->n_env * s->cluster_wide), "work")))
         err = 1;
     } else {
-      if (bad(env_occupancy(s->prec, s->material, s->fmt, s->tpv, s->threads, s->smem_bytes,
-                            s->cluster, &occ),
-              "occupancy"))
+      if (bad(block_occupancy(s, s->threads, s->cluster, &occ), "occupancy"))
         err = 1;
       s->capacity_blocks = s->cluster > 1 ? occ * s->cluster : occ * sms;
     }
@@ -1487,6 +1914,7 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
   const DevMesh m = s->mesh();
   cudaStream_t st = s->stream;
   int launches = 0;
+  if (s->by_domains) s->dom_seq = s->dom_seq + 1 < (1u << 28) ? s->dom_seq + 1 : 1;
   if (s->mode == VBD_MODE_BLOCK) {
     const double* dtol = nullptr;
     if (tol_env) {
@@ -1510,8 +1938,8 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
     NvtxRange nk("vbd_step_kernels");
     if (!s->tiered) {
       ++launches;
-      CUDA_TRY(launch_env_step(s->prec, s->material, s->tpv, s->threads, m, s->cur_params, dtol,
-                               s->d_work.p, (int)s->work.size(), s->cluster, s->smem_bytes, st));
+      CUDA_TRY(launch_block(s, m, s->cur_params, dtol, s->d_work.p, (int)s->work.size(), s->cluster,
+                            s->threads, s->smem_bytes, st));
     } else {
       // the launches with the widest clusters first (they need whole groups
       // of free SMs): wide tier, split environments, then the single-block
@@ -1544,8 +1972,8 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
         if (k >= 0) CUDA_TRY(cudaStreamWaitEvent(ts, s->ev_fork, 0));
         StepParams lp = s->cur_params;
         if (lp.trace) lp.trace += 4 * trace_off;
-        CUDA_TRY(launch_env_step(s->prec, s->material, s->tpv, t.threads, m, lp, dtol, t.dw,
-                                 (int)t.w->size(), t.cluster, t.smem, ts));
+        CUDA_TRY(launch_block(s, m, lp, dtol, t.dw, (int)t.w->size(), t.cluster, t.threads, t.smem,
+                              ts));
         if (k >= 0) CUDA_TRY(cudaEventRecord(side_join[k], ts));
         ++k;
         trace_off += t.w->size();
@@ -1564,11 +1992,16 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
     CUDA_TRY(cudaEventRecord(s->ev_k0, st));
     NvtxRange nk("vbd_step_kernels");
     ++launches;
-    PersistNbr nbr{};
-    if (s->persist_scoped) nbr = PersistNbr{s->d_nbr_off.p, s->d_nbr_idx.p, s->d_epoch.p};
-    CUDA_TRY(launch_persist(s->prec, s->material, s->tpv, s->threads, m, s->d_params.p,
-                            s->d_pctl.p, s->persist_blocks, s->wait_limits, s->d_pparts.p,
-                            s->persist_smem, nbr, st));
+    if (s->by_domains) {
+      CUDA_TRY(launch_domain(s->material, s->dom_tpv, s->threads, m, s->cur_params, dom_dev(s),
+                             nullptr, s->wait_limits, s->ndom, 1, true, s->dom_smem[0][0], st));
+    } else {
+      PersistNbr nbr{};
+      if (s->persist_scoped) nbr = PersistNbr{s->d_nbr_off.p, s->d_nbr_idx.p, s->d_epoch.p};
+      CUDA_TRY(launch_persist(s->prec, s->material, s->tpv, s->threads, m, s->d_params.p,
+                              s->d_pctl.p, s->persist_blocks, s->wait_limits, s->d_pparts.p,
+                              s->persist_smem, nbr, st));
+    }
   } else if (s->mode == VBD_MODE_GRAPH) {
     rc = build_graph(s);
     if (rc != VBD_OK) return rc;
