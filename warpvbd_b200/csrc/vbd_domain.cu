@@ -137,10 +137,11 @@ struct ChunkRegs {
   const ushort4* slot;
   int steps, lv, k, gv;
   bool valid, mailed;
-  double4 tt;
+  double4 tt;   // SPLIT: the vertex's inertia target and mass
+  int touched;  // else one word of it, to bring it into L1
 };
 
-template <int TPV>
+template <int TPV, bool SPLIT>
 __device__ __forceinline__ void load_chunk(ChunkRegs<TPV>& r, const DevMesh& m, const DomDev& d,
                                            const int4* chunk, const int2* local, int q,
                                            int lane) {
@@ -157,12 +158,19 @@ __device__ __forceinline__ void load_chunk(ChunkRegs<TPV>& r, const DevMesh& m, 
   r.mailed = false;
   r.gv = 0;
   r.tt = make_double4(0.0, 0.0, 0.0, 0.0);
+  r.touched = 0;
   if (r.valid) {
     const int2 o = local[r.lv];
     r.mailed = o.x < 0;
     r.gv = o.x < 0 ? ~o.x : o.x;
     r.k = o.y;
-    if (lane < CPW) r.tt = ldcg4(reinterpret_cast<const double4*>(m.ut) + r.gv);
+    const double4* tt = reinterpret_cast<const double4*>(m.ut) + r.gv;
+    if (lane < CPW) {
+      if (SPLIT)
+        r.tt = ldcg4(tt);
+      else
+        r.touched = *reinterpret_cast<const int*>(tt);
+    }
   }
 }
 
@@ -222,7 +230,7 @@ __device__ __forceinline__ void vertex_sums(double (&g)[3], double (&h)[6], int 
 
 // One warp updates the chunk's vertices; the sums of a vertex are formed as
 // process_chunk forms them.
-template <int TPV, int MAT>
+template <int TPV, int MAT, bool SPLIT>
 __device__ __forceinline__ void run_chunk(const ChunkRegs<TPV>& r, const DevMesh& m,
                                           const DomDev& d, const DomInfo& di, double* sp,
                                           const RecTab<double>& tab, int lane,
@@ -231,7 +239,7 @@ __device__ __forceinline__ void run_chunk(const ChunkRegs<TPV>& r, const DevMesh
                                           unsigned long long* dxrec) {
   constexpr int CPW = 32 / TPV;
   const int sub = lane / CPW;
-  const MailState st{sp, r.mailed ? d.mail + 3 * (size_t)r.gv : nullptr, tag};
+  const MailState st{sp, SPLIT && r.mailed ? d.mail + 3 * (size_t)r.gv : nullptr, tag};
   bool valid = r.valid;
 #if VBD_CHECK_BOUNDS
   if (valid && ((unsigned)r.lv >= (unsigned)di.nown || (unsigned)r.gv >= (unsigned)m.n_vertices)) {
@@ -262,11 +270,20 @@ __device__ __forceinline__ void run_chunk(const ChunkRegs<TPV>& r, const DevMesh
     if (s * TPV + sub < k) visit(__ldg(r.slot + s * 32));
   add_identity(h, hI);
   vertex_sums<TPV>(g, h, lane);
-  if (valid && lane < CPW)
-    finish_vertex<double, double>(m, r.gv, r.lv, uo, r.tt, g, h, st, sc, cmax, stat, dxrec);
+  if (valid && lane < CPW) {
+    double4 tt = r.tt;
+    if (!SPLIT) {
+      asm volatile("" ::"r"(r.touched));
+      tt = reinterpret_cast<const double4*>(m.ut)[r.gv];
+    }
+    finish_vertex<double, double>(m, r.gv, r.lv, uo, tt, g, h, st, sc, cmax, stat, dxrec);
+  }
 }
 
-template <int TPV, int MAT>
+// SPLIT: the launch's environments may be split over several blocks.  Without it
+// the handoff leaves the kernel, and with it the registers that made the slot
+// loop spill (27K slots on one block: 79 -> 75.5 us per sweep).
+template <int TPV, int MAT, bool SPLIT>
 __global__ void __launch_bounds__(kDomMaxThreads)
     domain_kernel(DevMesh m, StepParams p, DomDev d, const double* __restrict__ tol_env,
                   PersistLimits lim) {
@@ -291,7 +308,7 @@ __global__ void __launch_bounds__(kDomMaxThreads)
   const int max_iter = p.max_iter;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int warp = tid >> 5, lane = tid & 31, nwarps = nt >> 5;
-  const int nd = di.nd, ncolors = di.ncolors;
+  const int nd = SPLIT ? di.nd : 1, ncolors = di.ncolors;
   double* sp = reinterpret_cast<double*>(dsmem);
   RecTab<double> tab{d.rec + 3 * (size_t)di.rbase, nullptr};
   if (di.flags & kDomRecords) {
@@ -478,7 +495,7 @@ __global__ void __launch_bounds__(kDomMaxThreads)
   DomColor cc{};
   if (ncolors > 0) cc = s_color[0];
   if (cc.chunk_begin + warp < cc.chunk_end)
-    load_chunk<TPV>(r, m, d, chunk, local, cc.chunk_begin + warp, lane);
+    load_chunk<TPV, SPLIT>(r, m, d, chunk, local, cc.chunk_begin + warp, lane);
   if (ncolors == 0) {  // nothing is solved: no update, a largest one of zero
     conv = 0.0 < tol;
     it = conv ? 1 : max_iter;
@@ -496,15 +513,15 @@ __global__ void __launch_bounds__(kDomMaxThreads)
           if (lane < 2 * n.y)
             touch = __ldg(reinterpret_cast<const int*>(d.slot + (size_t)n.x * 32 + lane * 16));
         }
-        if (q != cc.chunk_begin + warp) load_chunk<TPV>(r, m, d, chunk, local, q, lane);
-        run_chunk<TPV, MAT>(r, m, d, di, sp, tab, lane, sc, tag, cmax, stat, dxrec);
+        if (q != cc.chunk_begin + warp) load_chunk<TPV, SPLIT>(r, m, d, chunk, local, q, lane);
+        run_chunk<TPV, MAT, SPLIT>(r, m, d, di, sp, tab, lane, sc, tag, cmax, stat, dxrec);
         asm volatile("" ::"r"(touch));
       }
       // the next colour's first chunk, then the wait for this one's halo
       const DomColor done = cc;
       cc = s_color[c + 1 < ncolors ? c + 1 : 0];
       if (cc.chunk_begin + warp < cc.chunk_end)
-        load_chunk<TPV>(r, m, d, chunk, local, cc.chunk_begin + warp, lane);
+        load_chunk<TPV, SPLIT>(r, m, d, chunk, local, cc.chunk_begin + warp, lane);
       const bool last = c + 1 == ncolors;
       if (last) {
         cmax = warp_max_u64(cmax);
@@ -598,28 +615,33 @@ __global__ void __launch_bounds__(kDomMaxThreads)
   }
 }
 
-template <typename F>
-cudaError_t dom_dispatch(int material, int tpv, F& f) {
-#define VBD_DOM_CASE(T) \
-  case T: return material == kSNH ? f.template run<T, kSNH>() : f.template run<T, kStVK>()
-  switch (tpv) {
-    VBD_DOM_CASE(2);
-    VBD_DOM_CASE(4);
-    VBD_DOM_CASE(8);
-    VBD_DOM_CASE(16);
-    VBD_DOM_CASE(32);
-    default: return cudaErrorInvalidValue;
-  }
-#undef VBD_DOM_CASE
+template <int TPV, typename F>
+cudaError_t dom_dispatch(int material, bool split, F& f) {
+  if (split)
+    return material == kSNH ? f.template run<TPV, kSNH, true>() : f.template run<TPV, kStVK, true>();
+  return material == kSNH ? f.template run<TPV, kSNH, false>()
+                          : f.template run<TPV, kStVK, false>();
 }
 
-template <int TPV, int MAT>
+template <typename F>
+cudaError_t dom_dispatch(int material, int tpv, bool split, F& f) {
+  switch (tpv) {
+    case 2: return dom_dispatch<2>(material, split, f);
+    case 4: return dom_dispatch<4>(material, split, f);
+    case 8: return dom_dispatch<8>(material, split, f);
+    case 16: return dom_dispatch<16>(material, split, f);
+    case 32: return dom_dispatch<32>(material, split, f);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+template <int TPV, int MAT, bool SPLIT>
 cudaError_t dom_configure() {
   static int configured_device = -1;  // the attributes are per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_device == dev) return cudaSuccess;
-  auto* k = domain_kernel<TPV, MAT>;
+  auto* k = domain_kernel<TPV, MAT, SPLIT>;
   cudaError_t e =
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDomMaxSmem);
   if (e == cudaSuccess)
@@ -633,12 +655,12 @@ struct DomOccupancy {
   size_t smem;
   int cluster;
   int* out;
-  template <int TPV, int MAT>
+  template <int TPV, int MAT, bool SPLIT>
   cudaError_t run() {
-    const cudaError_t e = dom_configure<TPV, MAT>();
+    const cudaError_t e = dom_configure<TPV, MAT, SPLIT>();
     if (e != cudaSuccess) return e;
     if (cluster <= 1)
-      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, domain_kernel<TPV, MAT>, threads,
+      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, domain_kernel<TPV, MAT, SPLIT>, threads,
                                                            smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster * 64);
@@ -651,7 +673,7 @@ struct DomOccupancy {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaOccupancyMaxActiveClusters(out, domain_kernel<TPV, MAT>, &cfg);
+    return cudaOccupancyMaxActiveClusters(out, domain_kernel<TPV, MAT, SPLIT>, &cfg);
   }
 };
 
@@ -666,9 +688,9 @@ struct DomLaunch {
   bool cooperative;
   size_t smem;
   cudaStream_t s;
-  template <int TPV, int MAT>
+  template <int TPV, int MAT, bool SPLIT>
   cudaError_t run() {
-    const cudaError_t e = dom_configure<TPV, MAT>();
+    const cudaError_t e = dom_configure<TPV, MAT, SPLIT>();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_blocks);
@@ -688,16 +710,17 @@ struct DomLaunch {
       attr[0].val.clusterDim.z = 1;
       cfg.numAttrs = 1;
     }
-    return cudaLaunchKernelEx(&cfg, domain_kernel<TPV, MAT>, m, p, d, tol, lim);
+    return cudaLaunchKernelEx(&cfg, domain_kernel<TPV, MAT, SPLIT>, m, p, d, tol, lim);
   }
 };
 
 }  // namespace
 
-cudaError_t dom_occupancy(int material, int tpv, int threads, size_t smem, int cluster, int* out) {
+cudaError_t dom_occupancy(int material, int tpv, int threads, size_t smem, int cluster,
+                          bool split, int* out) {
   if (threads < 32 || threads > kDomMaxThreads || threads % 32) return cudaErrorInvalidValue;
   DomOccupancy f{threads, smem, cluster, out};
-  return dom_dispatch(material, tpv, f);
+  return dom_dispatch(material, tpv, split, f);
 }
 
 cudaError_t launch_domain(int material, int tpv, int threads, const DevMesh& m,
@@ -708,7 +731,7 @@ cudaError_t launch_domain(int material, int tpv, int threads, const DevMesh& m,
       cluster < 1 || n_blocks % cluster || smem > kDomMaxSmem)
     return cudaErrorInvalidValue;
   DomLaunch f{threads, m, p, d, tol_env, lim, n_blocks, cluster, cooperative, smem, s};
-  return dom_dispatch(material, tpv, f);
+  return dom_dispatch(material, tpv, cluster > 1 || cooperative, f);
 }
 
 }  // namespace vbd

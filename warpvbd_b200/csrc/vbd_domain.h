@@ -86,8 +86,10 @@ inline size_t dom_smem(int nloc, int nrec, int nchunk, int flags) {
 // static arrays.
 constexpr size_t kDomMaxSmem = 227 * 1024 - 6400;
 
-// Resident blocks per SM (cluster = 1) or resident clusters on the device.
-cudaError_t dom_occupancy(int material, int tpv, int threads, size_t smem, int cluster, int* out);
+// Resident blocks per SM (cluster = 1) or resident clusters on the device; split:
+// of a launch with environments split over several blocks.
+cudaError_t dom_occupancy(int material, int tpv, int threads, size_t smem, int cluster,
+                          bool split, int* out);
 
 // One launch of a time step: n_blocks blocks, co-resident as a whole
 // (cooperative) or cluster by cluster.  Writes iters, status and the state of

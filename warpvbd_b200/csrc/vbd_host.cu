@@ -1335,7 +1335,8 @@ DomDev dom_dev(const vbd_solver* s) {
 // kernel at the solver's largest shared memory.
 cudaError_t block_occupancy(const vbd_solver* s, int threads, int cluster, int* out) {
   return s->by_domains
-             ? dom_occupancy(s->material, s->dom_tpv, threads, s->smem_bytes, cluster, out)
+             ? dom_occupancy(s->material, s->dom_tpv, threads, s->smem_bytes, cluster, cluster > 1,
+                             out)
              : env_occupancy(s->prec, s->material, s->fmt, s->tpv, threads, s->smem_bytes, cluster,
                              out);
 }
@@ -1641,7 +1642,8 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
                           s->dom_smem[i]);
     int resident = 0;
     if (D.fits && !block_mode) {
-      if (bad(dom_occupancy(s->material, s->dom_tpv, s->threads, s->dom_smem[0][0], 1, &resident),
+      if (bad(dom_occupancy(s->material, s->dom_tpv, s->threads, s->dom_smem[0][0], 1, true,
+                            &resident),
               "persist occupancy"))
         err = 1;
     }
