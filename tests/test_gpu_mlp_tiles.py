@@ -1,0 +1,25 @@
+"""The register-tiled forward pass at the edges of its tiles (64 and 128 samples), of the
+choice between them and on rows that are not 16-byte aligned, against fp64 numpy."""
+import numpy as np
+import pytest
+
+from oracle import mlp_oracle as mo
+from warpvbd_b200 import warmstart as ws
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 130, 148 * 256 - 1, 148 * 256, 148 * 256 + 129])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_forward_tiles(n, offset):
+    import torch
+    p = ws.init_params(1)
+    tr = ws.MLPTrainer(p, max_batch=64)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    flat = torch.randn(n * ws.FEAT_WIDTH + offset, device="cuda", generator=g)
+    X = flat[offset:].view(n, ws.FEAT_WIDTH)
+    out = tr.forward(X).cpu().numpy()
+    ref = mo.forward(p.astype(np.float64), X[:, :ws.N_IN].cpu().numpy().astype(np.float64))
+    ref = ref[0] if isinstance(ref, tuple) else ref
+    # three layers of at most 64 fp32 roundings (2^-24 each) of values of the result's size
+    assert np.abs(out - ref).max() < 3 * 64 * 2.0 ** -24 * max(1.0, np.abs(ref).max())
