@@ -462,9 +462,10 @@ __device__ __forceinline__ bool solve3(const double* h, const double* g, double*
   const double det = dot3(h[0], c00, h[1], c01, h[2], c02);
   if (!(fabs(det) > 1e-250 && fabs(det) < 1e250)) return chol_solve3<double>(h, g, x);
   const double r = -reciprocal64(det);
-  x[0] = dot3(c00, g[0], c01, g[1], c02, g[2]) * r;
-  x[1] = dot3(c01, g[0], c11, g[1], c12, g[2]) * r;
-  x[2] = dot3(c02, g[0], c12, g[1], c22, g[2]) * r;
+  // products the caller adds to: kept from being fused into those additions
+  x[0] = __dmul_rn(dot3(c00, g[0], c01, g[1], c02, g[2]), r);
+  x[1] = __dmul_rn(dot3(c01, g[0], c11, g[1], c12, g[2]), r);
+  x[2] = __dmul_rn(dot3(c02, g[0], c12, g[1], c22, g[2]), r);
   return (h[0] > 0.0) && (c22 > 0.0) && (det > 0.0);
 }
 __device__ __forceinline__ bool solve3(const float* h, const float* g, float* x) {
@@ -615,9 +616,10 @@ __device__ __forceinline__ void finish_vertex(const DevMesh& m, int gv, int lv,
                                               const StepConst& sc, unsigned long long& cmax,
                                               unsigned& stat, unsigned long long* dxrec) {
   using S4 = real4<SReal>;
-  const Real mdt2 = Real(tt.w * SReal(sc.inv_dt2));
+  Real mdt2 = Real(tt.w * SReal(sc.inv_dt2));
   Real G[3], H[6];
   if constexpr (sizeof(Real) == 8) {
+    mdt2 = __dmul_rn(tt.w, sc.inv_dt2);
     G[0] = fma(mdt2, uo.x - tt.x, g[0]);
     G[1] = fma(mdt2, uo.y - tt.y, g[1]);
     G[2] = fma(mdt2, uo.z - tt.z, g[2]);
@@ -641,7 +643,12 @@ __device__ __forceinline__ void finish_vertex(const DevMesh& m, int gv, int lv,
       G[2] += kd * (h[2] * ex + h[4] * ey + h[5] * ez);
     }
 #pragma unroll
-    for (int i = 0; i < 6; ++i) h[i] *= (Real(1) + kd);
+    for (int i = 0; i < 6; ++i) {
+      if constexpr (sizeof(Real) == 8)
+        h[i] = __dmul_rn(h[i], 1.0 + kd);
+      else
+        h[i] *= (Real(1) + kd);
+    }
   }
   H[0] = h[0] + mdt2;
   H[1] = h[1];

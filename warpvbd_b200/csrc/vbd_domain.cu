@@ -101,6 +101,7 @@ __device__ __forceinline__ bool wait_tagged(const ulonglong2* p, unsigned long l
 // Local state in shared memory; a store also mails a vertex other domains read.
 struct MailState {
   double* p;
+  double* save;  // where a store first puts the old position, or null
   ulonglong2* mail;  // the vertex's place, or null
   unsigned long long tag;
   __device__ __forceinline__ double4 load(int i) const {
@@ -111,6 +112,11 @@ struct MailState {
       st_tagged(mail, (unsigned long long)__double_as_longlong(v.x), tag);
       st_tagged(mail + 1, (unsigned long long)__double_as_longlong(v.y), tag);
       st_tagged(mail + 2, (unsigned long long)__double_as_longlong(v.z), tag);
+    }
+    if (save) {
+      save[3 * i] = p[3 * i];
+      save[3 * i + 1] = p[3 * i + 1];
+      save[3 * i + 2] = p[3 * i + 2];
     }
     p[3 * i] = v.x;
     p[3 * i + 1] = v.y;
@@ -232,14 +238,14 @@ __device__ __forceinline__ void vertex_sums(double (&g)[3], double (&h)[6], int 
 // process_chunk forms them.
 template <int TPV, int MAT, bool SPLIT>
 __device__ __forceinline__ void run_chunk(const ChunkRegs<TPV>& r, const DevMesh& m,
-                                          const DomDev& d, const DomInfo& di, double* sp,
+                                          const DomDev& d, const DomInfo& di, double* sp, double* save,
                                           const RecTab<double>& tab, int lane,
                                           const StepConst& sc, unsigned long long tag,
                                           unsigned long long& cmax, unsigned& stat,
                                           unsigned long long* dxrec) {
   constexpr int CPW = 32 / TPV;
   const int sub = lane / CPW;
-  const MailState st{sp, SPLIT && r.mailed ? d.mail + 3 * (size_t)r.gv : nullptr, tag};
+  const MailState st{sp, SPLIT ? save : nullptr, SPLIT && r.mailed ? d.mail + 3 * (size_t)r.gv : nullptr, tag};
   bool valid = r.valid;
 #if VBD_CHECK_BOUNDS
   if (valid && ((unsigned)r.lv >= (unsigned)di.nown || (unsigned)r.gv >= (unsigned)m.n_vertices)) {
@@ -366,7 +372,8 @@ __global__ void __launch_bounds__(kDomMaxThreads)
   };
   // every block's post of the next exchange into s_post, their status bits into
   // s_stat; false when a wait expired.  Followed by a block barrier.
-  auto collect = [&]() {
+  // seen: the largest value this thread read, instead
+  auto collect = [&](unsigned long long* seen = nullptr) {
     ++ex;
     bool ok = true;
     unsigned bits = 0u;
@@ -374,7 +381,10 @@ __global__ void __launch_bounds__(kDomMaxThreads)
       ulonglong2 got;
       ok = wait_tagged<8>(d.post + di.pbase + (int)(ex & 1) * nd + b, seq | ex, got, d, lim);
       if (!ok) break;
-      s_post[b] = got.x;
+      if (seen)
+        *seen = got.x > *seen ? got.x : *seen;
+      else
+        s_post[b] = got.x;
       bits |= (unsigned)(got.y & 0xffu);
     }
     bits = __reduce_or_sync(0xffffffffu, bits);
@@ -408,7 +418,7 @@ __global__ void __launch_bounds__(kDomMaxThreads)
   if (p.warm && m.ws_pred) {
     // as the block mode's stage: the incremental potential at the inertia guess
     // against inertia guess + alpha x prediction, alpha = 1, 1/2, 1/4
-    const MailState st{sp, nullptr, 0ull};
+    const MailState st{sp, nullptr, nullptr, 0ull};
     auto pred = [&](int l) { return m.ws_pred[local_gid(l)]; };
     auto moved = [&](double4 v, int l) {
       const float4 c = pred(l);
@@ -500,11 +510,41 @@ __global__ void __launch_bounds__(kDomMaxThreads)
     conv = 0.0 < tol;
     it = conv ? 1 : max_iter;
   }
+  // The answer of the convergence test, posted at a sweep's end, takes a trip
+  // through L2: the next sweep's first colour is computed meanwhile, its old
+  // positions kept in `save` in case the answer is to stop.  Not before the last
+  // sweep allowed, whose updates leave a record (dxrec).
+  double* save = reinterpret_cast<double*>(
+      dsmem + dom_smem_save(di.nloc, di.nrec, di.nchunk, di.flags));
+  const bool can_save = SPLIT && (di.flags & kDomSave) && !d.grid_sync;
+  bool asked = false;  // posted, answer not read yet
+  // every thread votes on the posts it read: all below the tolerance (a NaN, whose
+  // bits lie above infinity's, is not), or else something wrong.  False: aborted
+  auto answer = [&](bool ok) {
+    unsigned long long v = 0ull;
+    ok = collect(&v) && ok;
+    asked = false;
+    conv = __syncthreads_and(ok && __longlong_as_double((long long)v) < tol) != 0;
+    if (conv) return true;
+    if (__syncthreads_or(!ok)) return false;
+    nan = __syncthreads_or(v > 0x7ff0000000000000ull) != 0;
+    return true;
+  };
   while (ncolors > 0) {
     unsigned long long cmax = 0ull;
     unsigned long long* dxrec = it + 1 == max_iter ? m.dxmax + di.env : nullptr;
     const unsigned long long tag = seq | (unsigned long long)(it + 1);
+    bool undo = false;
     for (int c = 0; c < ncolors; ++c) {
+      // Warps of one scheduler start a colour 250 cycles apart: together they
+      // would all read their first slots and then all wait for the fp64 pipe,
+      // step after step (160x16x16 beam 33.2 -> 31.3 us per sweep, 27K slots on
+      // one block 75.3 -> 72.8; 150 and 350 cycles within 1 %)
+      if (cc.chunk_end - cc.chunk_begin > 4 && warp >= 4) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 250 * (warp >> 2 & 3)) {
+        }
+      }
       for (int q = cc.chunk_begin + warp; q < cc.chunk_end; q += nwarps) {
         // bring the slots of the warp's next chunk of this colour into L1
         int touch = 0;
@@ -514,7 +554,8 @@ __global__ void __launch_bounds__(kDomMaxThreads)
             touch = __ldg(reinterpret_cast<const int*>(d.slot + (size_t)n.x * 32 + lane * 16));
         }
         if (q != cc.chunk_begin + warp) load_chunk<TPV, SPLIT>(r, m, d, chunk, local, q, lane);
-        run_chunk<TPV, MAT, SPLIT>(r, m, d, di, sp, tab, lane, sc, tag, cmax, stat, dxrec);
+        run_chunk<TPV, MAT, SPLIT>(r, m, d, di, sp, asked ? save : nullptr, tab, lane, sc, tag,
+                                   cmax, stat, dxrec);
         asm volatile("" ::"r"(touch));
       }
       // the next colour's first chunk, then the wait for this one's halo
@@ -523,8 +564,20 @@ __global__ void __launch_bounds__(kDomMaxThreads)
       if (cc.chunk_begin + warp < cc.chunk_end)
         load_chunk<TPV, SPLIT>(r, m, d, chunk, local, cc.chunk_begin + warp, lane);
       const bool last = c + 1 == ncolors;
+      if (asked) {  // c == 0: the previous sweep's answer
+        if (!answer(last || receive(done, tag))) return abort_step();
+        undo = conv || nan;
+        if (undo) break;
+        if (!last) continue;
+      }
       if (last) {
-        cmax = warp_max_u64(cmax);
+        // only the lanes below CPW updated vertices
+        constexpr int CPW = 32 / TPV;
+#pragma unroll
+        for (int off = CPW / 2; off > 0; off >>= 1) {
+          const unsigned long long o = __shfl_xor_sync(0xffffffffu, cmax, off);
+          cmax = o > cmax ? o : cmax;
+        }
         const unsigned bits = __reduce_or_sync(0xffffffffu, stat);
         if (lane == 0) {
           s_red[it & 1][warp] = cmax;
@@ -549,19 +602,27 @@ __global__ void __launch_bounds__(kDomMaxThreads)
         if (tid == 0) post(0ull, 0u);
         ok = collect() && ok;
       }
-      if (last) ok = collect() && ok;
-      if (!__syncthreads_and(ok)) return abort_step();
+      if (last && !(can_save && it + 2 < max_iter)) {
+        if (!answer(ok)) return abort_step();
+      } else {
+        if (!__syncthreads_and(ok)) return abort_step();
+        asked = last;
+      }
     }
-    unsigned long long v = 0ull;
-    if (nd == 1) {
-      v = lane < nwarps ? s_red[it & 1][lane] : 0ull;
-    } else {
-      for (int b = lane; b < nd; b += 32) v = s_post[b] > v ? s_post[b] : v;
+    if (undo) {
+      // the last finished sweep's positions; `end` below reads each entry with the
+      // thread that restores it
+      for (int l = tid; l < di.nsave; l += nt)
+        for (int x = 0; x < 3; ++x) sp[3 * l + x] = save[3 * l + x];
+      break;
     }
-    v = warp_max_u64(v);
     ++it;
-    nan = v > 0x7ff0000000000000ull;
-    conv = !nan && __longlong_as_double((long long)v) < tol;
+    if (nd == 1) {
+      const unsigned long long v =
+          warp_max_u64(lane < nwarps ? s_red[(it - 1) & 1][lane] : 0ull);
+      nan = v > 0x7ff0000000000000ull;
+      conv = !nan && __longlong_as_double((long long)v) < tol;
+    }
     if (conv || nan || it >= max_iter) break;
   }
 

@@ -21,12 +21,15 @@ struct DomInfo {
   int qbase, nchunk;   // its chunks
   int cbase, ncolors;  // its colours
   int pbase;           // the environment's posts in DomDev::post: [2][nd]
-  int flags;           // kDomRecords, kDomMeta
+  int nsave;           // kDomSave: its vertices of the first colour
+  int flags;           // kDomRecords, kDomMeta, kDomSave
 };
 
 // What a block stages in shared memory beside the positions (else it reads
-// global memory): the records; the chunks and DomDev::local.
-constexpr int kDomRecords = 1, kDomMeta = 2;
+// global memory): the records; the chunks and DomDev::local.  kDomSave (all of an
+// environment's domains or none): room for the positions of the first colour,
+// which its next sweep starts on before the convergence test's answer is there.
+constexpr int kDomRecords = 1, kDomMeta = 2, kDomSave = 4;
 
 // One colour of one domain.
 struct DomColor {
@@ -70,17 +73,20 @@ constexpr int kDomMaxColors = 256;  // as the colouring's limit
 // Threads of a block at most; one block per SM.
 constexpr int kDomMaxThreads = 512;
 
-// Dynamic shared memory of a domain's block: positions, records, then chunks and
-// DomDev::local entries, each part only when staged.
+// Dynamic shared memory of a domain's block: positions, records, chunks and
+// DomDev::local entries, saved positions, each part only when its flag is set.
 __host__ __device__ inline size_t dom_smem_records(int nloc) {
   return ((size_t)nloc * 24 + 15) / 16 * 16;
 }
 __host__ __device__ inline size_t dom_smem_meta(int nloc, int nrec, int flags) {
   return dom_smem_records(nloc) + ((flags & kDomRecords) ? (size_t)nrec * 96 : 0);
 }
-inline size_t dom_smem(int nloc, int nrec, int nchunk, int flags) {
+__host__ __device__ inline size_t dom_smem_save(int nloc, int nrec, int nchunk, int flags) {
   return dom_smem_meta(nloc, nrec, flags) +
          ((flags & kDomMeta) ? (size_t)nchunk * 16 + (size_t)nloc * 8 : 0);
+}
+inline size_t dom_smem(int nloc, int nrec, int nchunk, int nsave, int flags) {
+  return dom_smem_save(nloc, nrec, nchunk, flags) + ((flags & kDomSave) ? (size_t)nsave * 24 : 0);
 }
 // Largest dynamic shared memory a domain may take: 227 KB less the kernel's
 // static arrays.

@@ -1185,6 +1185,7 @@ void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, i
   for (int t = e.tbase; t < e.tbase + e.ntets; ++t) tets[owner[L.tet_owner[t]]].push_back(t);
   std::vector<char> mailed(ns, 0);
   std::vector<int> loc(V, -1), rec_loc(e.nrec, -1), others, recs;
+  bool save = ndom > 1;
   for (int r = 0; r < ndom; ++r) {
     DomInfo di{};
     di.env = k;
@@ -1268,8 +1269,11 @@ void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, i
     }
     // shared memory: the records first, then the chunk and vertex lists
     for (int f : {kDomRecords, kDomMeta})
-      if (dom_smem(di.nloc, di.nrec, di.nchunk, di.flags | f) <= kDomMaxSmem) di.flags |= f;
-    D.fits = D.fits && dom_smem(di.nloc, 0, 0, 0) <= kDomMaxSmem && di.nloc <= 65536 &&
+      if (dom_smem(di.nloc, di.nrec, di.nchunk, 0, di.flags | f) <= kDomMaxSmem) di.flags |= f;
+    while (di.nsave < di.nown && color[own[r][di.nsave]] == 0) ++di.nsave;
+    save = save && dom_smem(di.nloc, di.nrec, di.nchunk, di.nsave, di.flags | kDomSave) <=
+                       kDomMaxSmem;
+    D.fits = D.fits && dom_smem(di.nloc, 0, 0, 0, 0) <= kDomMaxSmem && di.nloc <= 65536 &&
              di.nrec <= 65536 / 4 && C <= kDomMaxColors;
     D.dom.push_back(di);
     for (int v : own[r]) loc[v] = -1;
@@ -1277,9 +1281,11 @@ void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, i
     for (int q : recs) rec_loc[q] = -1;
     if (!D.fits) return;
   }
-  for (const DomInfo& di : D.dom)
+  for (DomInfo& di : D.dom) {
+    if (save) di.flags |= kDomSave;
     for (int l = di.lbase; l < di.lbase + di.nown; ++l)
       if (mailed[D.local[l].x - e.vbase]) D.local[l].x = ~D.local[l].x;
+  }
 }
 
 // Every environment in `parts` domains, appended to D; first[env] = its first
@@ -1306,7 +1312,7 @@ void build_all_domains(const Layout& L, int ltpv, const double* X, int tpv, int 
   for (int k = 0; k < n; ++k) {
     first[k] = (int)D.dom.size();
     for (const DomInfo& di : each[k].dom)
-      smem[k] = std::max(smem[k], dom_smem(di.nloc, di.nrec, di.nchunk, di.flags));
+      smem[k] = std::max(smem[k], dom_smem(di.nloc, di.nrec, di.nchunk, di.nsave, di.flags));
     D.append(each[k]);
     each[k] = DomLayout();
   }
