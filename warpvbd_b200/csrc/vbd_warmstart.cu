@@ -354,18 +354,18 @@ __global__ void __launch_bounds__(kFwdThreads, 4) mlp_forward_kernel(const float
 // Training step, fused per tile of kTrainTile samples (one block): forward
 // with the activations kept in shared memory, the loss gradient, backward to
 // the pre-activation deltas, and the tile's partial weight gradients -- each
-// parameter's sum over the tile's samples.  A second kernel adds the tiles'
-// partials in a fixed order, so the gradient is the same on every run (no
+// parameter's sum over the tile's samples, in sample order.  A second kernel adds
+// the tiles' partials in tile order, so the gradient is the same on every run (no
 // atomics).
 //
 // All matrices lie sample-fastest in shared memory.  The hidden layers and the
 // layer-1 deltas are register-tiled products of 4 units x 2 samples a thread,
 // the weight gradients of 4 x 4 (layer 2) and 2 x 3 (layer 1) parameters a
-// thread, four samples to a 16-byte load, all in packed fp32x2 multiply-adds: with
-// one result a thread every multiply-add loaded both operands from shared memory,
-// half a million of them per tile.  A 4,096-row minibatch (gradient and Adam) on
-// B200: 54 -> 38 us with the torch calls around it (tile kernel 35 -> 20, sum of
-// the tiles 9 -> 5.7); the launches are half of what is left.
+// thread, four samples to a 16-byte load: with one result a thread every
+// multiply-add loaded both operands from shared memory, half a million of them per
+// tile.  Every sum keeps its order, so loss, gradient and parameters have the bits
+// they had.  A 4,096-row minibatch (gradient and Adam) on B200: 54 -> 39 us with the
+// torch calls around it (tile kernel 35 -> 20); the launches are half of what is left.
 // ---------------------------------------------------------------------------
 constexpr int kTrainTile = 32;
 constexpr int kTrainThreads = 256;
@@ -407,37 +407,28 @@ __device__ __forceinline__ void train_product(const float* WT, const float* a, i
   }
 }
 
-// Sums over the tile's samples of A[row][s] B[col][s] for NA x NB rows.
+// Sums over the tile's samples, in order, of A[row][s] B[col][s] for NA x NB rows.
 template <int NA, int NB>
 __device__ __forceinline__ void train_gradient(const float* A, int sa, const float* B, int sb,
                                                float (&r)[NA][NB]) {
-  f32x2 acc[NA][NB];
 #pragma unroll
   for (int i = 0; i < NA; ++i)
 #pragma unroll
-    for (int j = 0; j < NB; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < NB; ++j) r[i][j] = 0.0f;
 #pragma unroll 2
   for (int s = 0; s < kTrainTile; s += 4) {
-    ulonglong2 a[NA], b[NB];
+    float4 a[NA], b[NB];
 #pragma unroll
-    for (int i = 0; i < NA; ++i)
-      a[i] = *reinterpret_cast<const ulonglong2*>(A + i * sa * kTsPitch + s);
+    for (int i = 0; i < NA; ++i) a[i] = *reinterpret_cast<const float4*>(A + i * sa * kTsPitch + s);
 #pragma unroll
-    for (int j = 0; j < NB; ++j)
-      b[j] = *reinterpret_cast<const ulonglong2*>(B + j * sb * kTsPitch + s);
+    for (int j = 0; j < NB; ++j) b[j] = *reinterpret_cast<const float4*>(B + j * sb * kTsPitch + s);
 #pragma unroll
     for (int i = 0; i < NA; ++i)
 #pragma unroll
       for (int j = 0; j < NB; ++j)
-        acc[i][j] = fma2(a[i].y, b[j].y, fma2(a[i].x, b[j].x, acc[i][j]));
+        r[i][j] = fmaf(a[i].w, b[j].w,
+                       fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, r[i][j]))));
   }
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      const float2 v = unpack2(acc[i][j]);
-      r[i][j] = v.x + v.y;
-    }
 }
 
 __global__ void __launch_bounds__(kTrainThreads) mlp_train_tile_kernel(
@@ -532,8 +523,8 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_tile_kernel(
                   w2 = ts[kTsW3 + 2 * kWsHidden + u];
       const float2 g = *reinterpret_cast<const float2*>(ts + kTsG2 + at);
       *reinterpret_cast<float2*>(ts + kTsD2 + at) =
-          make_float2((w0 * o0.x + w1 * o1.x + w2 * o2.x) * g.x,
-                      (w0 * o0.y + w1 * o1.y + w2 * o2.y) * g.y);
+          make_float2(fmaf(w2, o2.x, fmaf(w1, o1.x, w0 * o0.x)) * g.x,
+                      fmaf(w2, o2.y, fmaf(w1, o1.y, w0 * o0.y)) * g.y);
     }
   }
   __syncthreads();
@@ -561,13 +552,13 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_tile_kernel(
       for (int j = 0; j < 4; ++j) dst[kWsW2 + (ty + 16 * i) * kWsHidden + tx + 16 * j] = r[i][j];
   }
   auto row_sum = [&](const float* row) {
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    float a = 0.0f;
 #pragma unroll
     for (int s = 0; s < kTrainTile; s += 4) {
       const float4 v = *reinterpret_cast<const float4*>(row + s);
-      a = make_float4(a.x + v.x, a.y + v.y, a.z + v.z, a.w + v.w);
+      a = (((a + v.x) + v.y) + v.z) + v.w;
     }
-    return (a.x + a.y) + (a.z + a.w);
+    return a;
   };
   if (t < kWsOut * kWsHidden) {  // W3[k][j] += dout[k][s] S2[j][s]
     float r[1][1];
@@ -597,38 +588,27 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_tile_kernel(
   }
 }
 
-// Sum of the tiles' partial gradients (and of their squared errors into *loss):
-// the tiles in four runs, each in order, and the runs in order.
-constexpr int kReduceCols = 64, kReduceRuns = 4;
-__global__ void __launch_bounds__(kReduceCols* kReduceRuns)
+// Sum of the tiles' partial gradients in tile order (and of their squared
+// errors into *loss): a parameter a thread, 32 tiles' partials in flight.
+constexpr int kReduceThreads = 64;
+__global__ void __launch_bounds__(kReduceThreads)
     mlp_reduce_tiles_kernel(const float* __restrict__ part, int tiles, float* __restrict__ grad,
                             double* __restrict__ loss) {
-  __shared__ float s_part[kReduceRuns][kReduceCols];
-  __shared__ double s_loss[kReduceRuns];
-  const int c = threadIdx.x % kReduceCols, run = threadIdx.x / kReduceCols;
-  const int p = blockIdx.x * kReduceCols + c;
-  const int per = (tiles + kReduceRuns - 1) / kReduceRuns;
-  const int b0 = run * per, b1 = min(tiles, b0 + per);
+  const int p = blockIdx.x * kReduceThreads + threadIdx.x;
+  if (p > kWsParams) return;
+  if (p == kWsParams) {
+    if (loss) {
+      double v = 0.0;
+#pragma unroll 32
+      for (int b = 0; b < tiles; ++b) v += double(part[(size_t)b * kTrainPartial + p]);
+      *loss += v;
+    }
+    return;
+  }
   float acc = 0.0f;
-  if (p < kWsParams) {
-#pragma unroll 8
-    for (int b = b0; b < b1; ++b) acc += part[(size_t)b * kTrainPartial + p];
-  } else if (p == kWsParams) {
-    double v = 0.0;
-    for (int b = b0; b < b1; ++b) v += double(part[(size_t)b * kTrainPartial + p]);
-    s_loss[run] = v;
-  }
-  s_part[run][c] = acc;
-  __syncthreads();
-  if (run != 0) return;
-  if (p < kWsParams) {
-    for (int i = 1; i < kReduceRuns; ++i) acc += s_part[i][c];
-    grad[p] = acc;
-  } else if (p == kWsParams && loss) {
-    double v = s_loss[0];
-    for (int i = 1; i < kReduceRuns; ++i) v += s_loss[i];
-    *loss += v;
-  }
+#pragma unroll 32
+  for (int b = 0; b < tiles; ++b) acc += part[(size_t)b * kTrainPartial + p];
+  grad[p] = acc;
 }
 
 __global__ void adam_kernel(float* __restrict__ P, const float* __restrict__ G,
@@ -718,7 +698,7 @@ cudaError_t launch_mlp_train_batch(const float* X, const float* Y, const int* id
   }
   const int tiles = nblk(batch, kTrainTile);
   mlp_train_tile_kernel<<<tiles, kTrainThreads, kTrainSmem, s>>>(X, Y, idx, batch, P, scratch);
-  mlp_reduce_tiles_kernel<<<nblk(kTrainPartial, kReduceCols), kReduceCols * kReduceRuns, 0, s>>>(
+  mlp_reduce_tiles_kernel<<<nblk(kTrainPartial, kReduceThreads), kReduceThreads, 0, s>>>(
       scratch, tiles, grad, loss);
   return cudaGetLastError();
 }
