@@ -1419,7 +1419,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     }
   }
   // mode / threads / tpv
-  const bool tpv_given = tpv != 0, threads_given = threads != 0;
+  const bool tpv_given = tpv != 0;
   int mode = flags & VBD_MODE_MASK;
   // provisional environment size bound for the shared-memory check
   int max_env_v = 0;
@@ -1639,7 +1639,9 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     // sweep of 27K slots)
     s->dom_tpv = tpv_given ? (s->n_env > 1 ? std::max(4, s->tpv) : s->tpv)
                            : (s->n_env > 1 ? 4 : domain_tpv(per));
-    if (!block_mode && !threads_given) s->threads = per <= 64 ? 256 : 512;
+    // one block per SM in persistent mode, whose warps are all the SM has: the
+    // thread count is the domains' (a given one was meant for several blocks per SM)
+    if (!block_mode) s->threads = per <= 64 ? 256 : 512;
     DomLayout D;
     std::vector<int> first[3];
     for (int i = 0; i < 3 && D.fits; ++i)
@@ -1687,6 +1689,8 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
         s->smem_bytes = 0;
         for (const auto& v : s->dom_smem)
           for (size_t x : v) s->smem_bytes = std::max(s->smem_bytes, x);
+        // blocks too large for two on an SM get the SM's warps
+        if (2 * (s->smem_bytes + 7 * 1024) > 227 * 1024) s->threads = kDomMaxThreads;
       }
     }
   }
