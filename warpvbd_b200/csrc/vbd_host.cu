@@ -16,8 +16,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -100,6 +102,36 @@ int greedy_coloring(const int32_t* tets, int T, int nv, int32_t* col) {
     ncol = std::max(ncol, c + 1);
   }
   return ncol;
+}
+
+// f(0) ... f(n - 1) on up to 16 host threads; an exception of f is rethrown here.
+template <class F>
+void for_each_parallel(int n, F f) {
+  std::atomic<int> next{0};
+  std::mutex mu;
+  std::exception_ptr error;
+  auto work = [&]() {
+    for (int k; (k = next.fetch_add(1)) < n;) {
+      try {
+        f(k);
+      } catch (...) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!error) error = std::current_exception();
+        next = n;
+      }
+    }
+  };
+  const int nthreads =
+      std::min<int>(n, std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
+  std::vector<std::thread> pool;
+  pool.reserve(nthreads);
+  try {
+    for (int i = 1; i < nthreads; ++i) pool.emplace_back(work);
+  } catch (const std::system_error&) {  // no more threads: those there are do it
+  }
+  work();
+  for (auto& t : pool) t.join();
+  if (error) std::rethrow_exception(error);
 }
 
 struct TetData {
@@ -226,262 +258,331 @@ struct Layout {
   long long n_slots = 0;
 };
 
-// `greedy`: the greedy colouring of the whole mesh, already computed (on the
-// GPU); every environment's colours are its slice (environments share no tet,
-// so a vertex's lower neighbours all lie in its environment).  Null: the
-// colouring is computed here per environment.
-int build_layout(const double* X, int V, const int32_t* tets, int T, const uint8_t* active,
-                 const std::vector<int>& voff, const std::vector<int>& toff,
-                 const int32_t* coloring, const TetData& td, int tpv, bool order_index,
-                 Layout& L, const int32_t* greedy = nullptr) {
-  const int n_env = (int)voff.size() - 1;
+// Environment e: its part of the per-vertex arrays of L (new_of_old, valence,
+// mass, wstat; environment 0 also the colour table), everything else appended to
+// P, whose offsets count from zero.  `greedy`: the greedy colouring of the whole
+// mesh, already computed (on the GPU); every environment's colours are its slice
+// (environments share no tet, so a vertex's lower neighbours all lie in its
+// environment).  Null: the colouring is computed here per environment.
+int build_env_layout(int e, int n_env, const int32_t* tets, const uint8_t* active,
+                     const std::vector<int>& voff, const std::vector<int>& toff,
+                     const int32_t* coloring, const TetData& td, int tpv, bool order_index,
+                     const int32_t* greedy, Layout& L, Layout& P) {
   const int cpw = 32 / tpv;
+  int block_count = 0;
+  const int vo = voff[e], vn = voff[e + 1] - voff[e];
+  const int to = toff[e], tn = toff[e + 1] - toff[e];
+  if (vn < 0 || tn < 0) return fail(VBD_ERR_INVALID_ARG, "environment offsets decrease");
+  std::vector<int32_t> lt(4 * (size_t)tn);
+  int nv_col = 0;
+  for (size_t i = 0; i < lt.size(); ++i) {
+    const int g = tets[4 * (size_t)to + i];
+    if (g < vo || g >= vo + vn)
+      return fail(VBD_ERR_INVALID_ARG, "tet " + std::to_string(to + i / 4) +
+                                           " references a vertex outside its environment");
+    lt[i] = g - vo;
+    nv_col = std::max(nv_col, lt[i] + 1);
+  }
+  // colours of the local vertices (-1: not coloured)
+  std::vector<int32_t> col(vn, -1);
+  int ncol = 0;
+  if (coloring && n_env == 1) {
+    for (int v = 0; v < nv_col; ++v) {
+      col[v] = coloring[v];
+      if (col[v] < 0 || col[v] >= 256) return fail(VBD_ERR_INVALID_ARG, "bad colour value");
+      ncol = std::max(ncol, col[v] + 1);
+    }
+    // vertices of one colour must not share a tet, or their updates race
+    for (int t = 0; t < tn; ++t)
+      for (int a = 0; a < 4; ++a)
+        for (int b = a + 1; b < 4; ++b)
+          if (col[lt[4 * (size_t)t + a]] == col[lt[4 * (size_t)t + b]])
+            return fail(VBD_ERR_INVALID_ARG,
+                        "coloring gives two vertices of tet " + std::to_string(t) +
+                            " the same colour");
+  } else if (tn > 0 && greedy) {
+    // as the per-environment pass colours them: ids 0 .. max local id
+    for (int v = 0; v < nv_col; ++v) {
+      col[v] = greedy[vo + v];
+      ncol = std::max(ncol, col[v] + 1);
+    }
+  } else if (tn > 0) {
+    ncol = greedy_coloring(lt.data(), tn, nv_col, col.data());
+    if (ncol < 0) return fail(VBD_ERR_TOO_MANY_COLORS, "Exceeded maximum number of colors");
+  }
+  // incident tets, ascending tet id
+  std::vector<int> off(vn + 1, 0), inc(4 * (size_t)tn), loc(4 * (size_t)tn);
+  for (size_t i = 0; i < lt.size(); ++i) off[lt[i] + 1]++;
+  for (int v = 0; v < vn; ++v) off[v + 1] += off[v];
+  {
+    std::vector<int> fill(off.begin(), off.end() - 1);
+    for (int t = 0; t < tn; ++t)
+      for (int q = 0; q < 4; ++q) {
+        const int v = lt[4 * (size_t)t + q];
+        inc[fill[v]] = t;
+        loc[fill[v]] = q;
+        fill[v]++;
+      }
+  }
+  // colour table of environment 0 in the reference layout
+  if (e == 0) {
+    std::vector<std::vector<int>> groups(ncol);
+    for (int v = 0; v < nv_col; ++v)
+      if (col[v] >= 0) groups[col[v]].push_back(vo + v);
+    int mg = 0;
+    for (auto& g : groups) mg = std::max(mg, (int)g.size());
+    L.table_colors = ncol;
+    L.table_max_group = mg;
+    L.table0.assign((size_t)ncol * mg, -1);
+    for (int c = 0; c < ncol; ++c)
+      for (size_t i = 0; i < groups[c].size(); ++i) L.table0[(size_t)c * mg + i] = groups[c][i];
+  }
+  // classify and order
+  std::vector<std::vector<int>> solved(ncol);
+  std::vector<int> freev, fixedv;
+  for (int v = 0; v < vn; ++v) {
+    const bool act = active ? active[vo + v] != 0 : true;
+    const int k = off[v + 1] - off[v];
+    if (!act)
+      fixedv.push_back(v);
+    else if (col[v] >= 0 && k > 0)
+      solved[col[v]].push_back(v);
+    else
+      freev.push_back(v);
+    P.max_valence = std::max(P.max_valence, k);
+  }
+  EnvInfo ei{};
+  ei.vbase = vo;
+  ei.nv = vn;
+  ei.cbase = (int)P.color.size();
+  int next = 0;
+  std::vector<int> new_local(vn, -1);
+  for (int c = 0; c < ncol; ++c) {
+    auto& g = solved[c];
+    if (g.empty()) continue;
+    if (!order_index)
+      std::stable_sort(g.begin(), g.end(), [&](int a, int b) {
+        return (off[a + 1] - off[a]) > (off[b + 1] - off[b]);
+      });
+    ColorInfo ci{};
+    ci.vbegin = vo + next;
+    for (int v : g) new_local[v] = next++;
+    ci.vend = vo + next;
+    ci.chunk_begin = (int)P.chunk.size();
+    const int ng = (int)g.size();
+    for (int base = 0; base < ng; base += cpw) {
+      int kmax = 0;
+      for (int i = base; i < std::min(ng, base + cpw); ++i)
+        kmax = std::max(kmax, off[g[i] + 1] - off[g[i]]);
+      ChunkInfo ch{};
+      ch.block = block_count;
+      ch.steps = (kmax + tpv - 1) / tpv;
+      block_count += ch.steps;
+      P.chunk.push_back(ch);
+    }
+    ci.chunk_end = (int)P.chunk.size();
+    P.color.push_back(ci);
+  }
+  ei.nsolved = next;
+  for (int v : freev) new_local[v] = next++;
+  ei.nact = next;
+  for (int v : fixedv) new_local[v] = next++;
+  ei.ncolors = (int)P.color.size() - ei.cbase;
+  P.env.push_back(ei);
+  P.max_colors = std::max(P.max_colors, ei.ncolors);
+  P.max_env_vertices = std::max(P.max_env_vertices, vn);
+  std::vector<double> edge(tn), log_e(tn);  // per tet: length scale, log10 E
+  for (int t = 0; t < tn; ++t) {
+    edge[t] = std::cbrt(6.0 * td.vol[to + t]);
+    log_e[t] = std::log10(td.E[to + t]);
+  }
+  for (int v = 0; v < vn; ++v) {
+    const int gnew = vo + new_local[v];
+    L.new_of_old[vo + v] = gnew;
+    const int k = off[v + 1] - off[v];
+    L.valence[gnew] = k;
+    double m = 0.0, hs = 0.0, logE = 0.0, rho = 0.0, nu = 0.0;
+    for (int s = off[v]; s < off[v + 1]; ++s) {
+      const int t = to + inc[s];
+      m += td.mass[t] / 4.0;
+      hs += edge[inc[s]];
+      logE += log_e[inc[s]];
+      rho += td.rho[t];
+      nu += td.nu[t];
+    }
+    L.mass[gnew] = m;
+    // warm-start vertex constants: local length scale h (mean cube root of
+    // 6 V over the incident tets), log10(E / (rho h^2)), nu, valence / 20
+    float* w4 = &L.wstat[4 * (size_t)gnew];
+    if (k > 0) {
+      const double h = hs / k;
+      w4[0] = (float)h;
+      w4[1] = (float)(logE / k - std::log10(rho / k * h * h));
+      w4[2] = (float)(nu / k);
+      w4[3] = (float)(k / 20.0);
+    } else {
+      w4[0] = 1.0f;
+      w4[1] = w4[2] = w4[3] = 0.0f;
+    }
+  }
+  for (int c = ei.cbase; c < ei.cbase + ei.ncolors; ++c)
+    for (int q = P.color[c].chunk_begin; q < P.color[c].chunk_end; ++q)
+      P.chunk_owner.push_back(make_int2(c, e));
+  // slot records: (n0, n1, n2, record id) per slot, the record values in a
+  // table of this environment shared by every slot with the same values in
+  // the solver precision (record ids are environment-local, so a block can
+  // stage its environment's table in shared memory)
+  P.rec_idx.resize((size_t)block_count * 32, make_int4(0, 0, 0, 0));
+  RecordTable etab;
+  etab.fp64 = P.table.fp64;
+  std::vector<int> tet_rec(etab.fp64 ? tn : 0, -1);  // fp64: record of each tet
+  std::vector<std::pair<int, int4>> tlist;  // (owner, owner slot) per tet
+  std::vector<int> old_of_new_local(vn);
+  for (int v = 0; v < vn; ++v) old_of_new_local[new_local[v]] = v;
+  for (int ci_i = ei.cbase; ci_i < ei.cbase + ei.ncolors; ++ci_i) {
+    const ColorInfo ci = P.color[ci_i];
+    for (int q = ci.chunk_begin; q < ci.chunk_end; ++q) {
+      const ChunkInfo ch = P.chunk[q];
+      for (int lane = 0; lane < 32; ++lane) {
+        const int vi = lane / tpv, sub = lane % tpv;
+        const int gv = ci.vbegin + (q - ci.chunk_begin) * cpw + vi;
+        if (gv >= ci.vend) continue;
+        const int ov = old_of_new_local[gv - vo];
+        const int k = off[ov + 1] - off[ov];
+        for (int s = 0; s < ch.steps; ++s) {
+          const int j = s * tpv + sub;
+          if (j >= k) break;
+          const int t = to + inc[off[ov] + j];
+          const int a = loc[off[ov] + j];
+          const size_t blk = (size_t)ch.block + s;
+          int ids[3];
+          const double* bt = &td.b[(size_t)t * 12];
+          const double* pt = &td.p[(size_t)t * 3];
+          int n = 0, solved_in_tet = 0, owner = vn;
+          for (int qq = 0; qq < 4; ++qq) {
+            const int nl = new_local[tets[4 * (size_t)t + qq] - vo];
+            if (nl < ei.nsolved) {
+              ++solved_in_tet;
+              owner = std::min(owner, nl);
+            }
+            if (qq != a) ids[n++] = nl;
+          }
+          int rid;
+          if (etab.fp64) {
+            int& rec = tet_rec[t - to];
+            if (rec < 0) {
+              double val[12];
+              for (int i = 0; i < 3; ++i) {
+                for (int c = 0; c < 3; ++c) val[4 * i + c] = bt[3 * i + c];
+                val[4 * i + 3] = pt[i & 1];
+              }
+              rec = etab.insert(val);
+            }
+            rid = 4 * rec + a;
+          } else {
+            double val[12];
+            n = 0;
+            for (int qq = 0; qq < 4; ++qq) {
+              if (qq == a) continue;
+              for (int c = 0; c < 3; ++c) val[4 * n + c] = bt[qq * 3 + c];
+              val[4 * n + 3] = pt[n];
+              ++n;
+            }
+            // 4th value of the last row: this slot's share of the tet's
+            // strain energy
+            val[11] = 1.0 / solved_in_tet;
+            rid = etab.insert(val);
+          }
+          P.rec_idx[blk * 32 + lane] = make_int4(ids[0], ids[1], ids[2], rid);
+          if (owner == gv - vo) tlist.emplace_back(owner, make_int4(ids[0], ids[1], ids[2], rid));
+          P.n_slots++;
+        }
+      }
+    }
+  }
+  P.env.back().rbase = P.table.size();
+  P.env.back().nrec = etab.size();
+  // the tet list in owner order (neighbouring entries read nearby state)
+  std::stable_sort(tlist.begin(), tlist.end(),
+                   [](const std::pair<int, int4>& a, const std::pair<int, int4>& b) {
+                     return a.first < b.first;
+                   });
+  P.env.back().tbase = (int)P.tet_slot.size();
+  P.env.back().ntets = (int)tlist.size();
+  for (const auto& x : tlist) {
+    P.tet_owner.push_back(x.first);
+    P.tet_slot.push_back(x.second);
+  }
+  P.table.vals.insert(P.table.vals.end(), etab.vals.begin(), etab.vals.end());
+  P.max_env_records = std::max(P.max_env_records, etab.size());
+  return VBD_OK;
+}
+
+// The whole layout.  The environments are independent: host threads take them in
+// turn, and their parts are joined in order.
+int build_layout(int V, const int32_t* tets, const uint8_t* active, const std::vector<int>& voff,
+                 const std::vector<int>& toff, const int32_t* coloring, const TetData& td, int tpv,
+                 bool order_index, Layout& L, const int32_t* greedy = nullptr) {
+  const int n_env = (int)voff.size() - 1;
   L.new_of_old.assign(V, -1);
   L.valence.assign(V, 0);
   L.mass.assign(V, 0.0);
   L.wstat.assign(4 * (size_t)V, 0.0f);
-  int block_count = 0;
+  std::vector<Layout> part(n_env);
+  std::vector<int> rc(n_env, VBD_OK);
+  std::vector<std::string> why(n_env);  // the message is per thread: carried over
+  for_each_parallel(n_env, [&](int e) {
+    part[e].table.fp64 = L.table.fp64;
+    rc[e] = build_env_layout(e, n_env, tets, active, voff, toff, coloring, td, tpv, order_index,
+                             greedy, L, part[e]);
+    if (rc[e] != VBD_OK) why[e] = g_last_error;
+  });
+  for (int e = 0; e < n_env; ++e)
+    if (rc[e] != VBD_OK) return fail(rc[e], why[e]);
+  if (n_env == 1) {  // nothing to join
+    Layout& P = part[0];
+    L.env.swap(P.env);
+    L.color.swap(P.color);
+    L.chunk.swap(P.chunk);
+    L.rec_idx.swap(P.rec_idx);
+    L.chunk_owner.swap(P.chunk_owner);
+    L.tet_slot.swap(P.tet_slot);
+    L.tet_owner.swap(P.tet_owner);
+    L.table.vals.swap(P.table.vals);
+  }
+  size_t slots = 0;
+  for (const Layout& P : part) slots += P.rec_idx.size();
+  L.rec_idx.reserve(std::max(L.rec_idx.size(), slots));
   for (int e = 0; e < n_env; ++e) {
-    const int vo = voff[e], vn = voff[e + 1] - voff[e];
-    const int to = toff[e], tn = toff[e + 1] - toff[e];
-    if (vn < 0 || tn < 0) return fail(VBD_ERR_INVALID_ARG, "environment offsets decrease");
-    std::vector<int32_t> lt(4 * (size_t)tn);
-    int nv_col = 0;
-    for (size_t i = 0; i < lt.size(); ++i) {
-      const int g = tets[4 * (size_t)to + i];
-      if (g < vo || g >= vo + vn)
-        return fail(VBD_ERR_INVALID_ARG, "tet " + std::to_string(to + i / 4) +
-                                             " references a vertex outside its environment");
-      lt[i] = g - vo;
-      nv_col = std::max(nv_col, lt[i] + 1);
+    Layout& P = part[e];
+    const int nc = (int)L.color.size(), nq = (int)L.chunk.size();
+    const int nb = (int)(L.rec_idx.size() / 32);
+    for (EnvInfo ei : P.env) {
+      ei.cbase += nc;
+      ei.rbase += L.table.size();
+      ei.tbase += (int)L.tet_slot.size();
+      L.env.push_back(ei);
     }
-    // colours of the local vertices (-1: not coloured)
-    std::vector<int32_t> col(vn, -1);
-    int ncol = 0;
-    if (coloring && n_env == 1) {
-      for (int v = 0; v < nv_col; ++v) {
-        col[v] = coloring[v];
-        if (col[v] < 0 || col[v] >= 256) return fail(VBD_ERR_INVALID_ARG, "bad colour value");
-        ncol = std::max(ncol, col[v] + 1);
-      }
-      // vertices of one colour must not share a tet, or their updates race
-      for (int t = 0; t < tn; ++t)
-        for (int a = 0; a < 4; ++a)
-          for (int b = a + 1; b < 4; ++b)
-            if (col[lt[4 * (size_t)t + a]] == col[lt[4 * (size_t)t + b]])
-              return fail(VBD_ERR_INVALID_ARG,
-                          "coloring gives two vertices of tet " + std::to_string(t) +
-                              " the same colour");
-    } else if (tn > 0 && greedy) {
-      // as the per-environment pass colours them: ids 0 .. max local id
-      for (int v = 0; v < nv_col; ++v) {
-        col[v] = greedy[vo + v];
-        ncol = std::max(ncol, col[v] + 1);
-      }
-    } else if (tn > 0) {
-      ncol = greedy_coloring(lt.data(), tn, nv_col, col.data());
-      if (ncol < 0) return fail(VBD_ERR_TOO_MANY_COLORS, "Exceeded maximum number of colors");
-    }
-    // incident tets, ascending tet id
-    std::vector<int> off(vn + 1, 0), inc(4 * (size_t)tn), loc(4 * (size_t)tn);
-    for (size_t i = 0; i < lt.size(); ++i) off[lt[i] + 1]++;
-    for (int v = 0; v < vn; ++v) off[v + 1] += off[v];
-    {
-      std::vector<int> fill(off.begin(), off.end() - 1);
-      for (int t = 0; t < tn; ++t)
-        for (int q = 0; q < 4; ++q) {
-          const int v = lt[4 * (size_t)t + q];
-          inc[fill[v]] = t;
-          loc[fill[v]] = q;
-          fill[v]++;
-        }
-    }
-    // colour table of environment 0 in the reference layout
-    if (e == 0) {
-      std::vector<std::vector<int>> groups(ncol);
-      for (int v = 0; v < nv_col; ++v)
-        if (col[v] >= 0) groups[col[v]].push_back(vo + v);
-      int mg = 0;
-      for (auto& g : groups) mg = std::max(mg, (int)g.size());
-      L.table_colors = ncol;
-      L.table_max_group = mg;
-      L.table0.assign((size_t)ncol * mg, -1);
-      for (int c = 0; c < ncol; ++c)
-        for (size_t i = 0; i < groups[c].size(); ++i) L.table0[(size_t)c * mg + i] = groups[c][i];
-    }
-    // classify and order
-    std::vector<std::vector<int>> solved(ncol);
-    std::vector<int> freev, fixedv;
-    for (int v = 0; v < vn; ++v) {
-      const bool act = active ? active[vo + v] != 0 : true;
-      const int k = off[v + 1] - off[v];
-      if (!act)
-        fixedv.push_back(v);
-      else if (col[v] >= 0 && k > 0)
-        solved[col[v]].push_back(v);
-      else
-        freev.push_back(v);
-      L.max_valence = std::max(L.max_valence, k);
-    }
-    EnvInfo ei{};
-    ei.vbase = vo;
-    ei.nv = vn;
-    ei.cbase = (int)L.color.size();
-    int next = 0;
-    std::vector<int> new_local(vn, -1);
-    for (int c = 0; c < ncol; ++c) {
-      auto& g = solved[c];
-      if (g.empty()) continue;
-      if (!order_index)
-        std::stable_sort(g.begin(), g.end(), [&](int a, int b) {
-          return (off[a + 1] - off[a]) > (off[b + 1] - off[b]);
-        });
-      ColorInfo ci{};
-      ci.vbegin = vo + next;
-      for (int v : g) new_local[v] = next++;
-      ci.vend = vo + next;
-      ci.chunk_begin = (int)L.chunk.size();
-      const int ng = (int)g.size();
-      for (int base = 0; base < ng; base += cpw) {
-        int kmax = 0;
-        for (int i = base; i < std::min(ng, base + cpw); ++i)
-          kmax = std::max(kmax, off[g[i] + 1] - off[g[i]]);
-        ChunkInfo ch{};
-        ch.block = block_count;
-        ch.steps = (kmax + tpv - 1) / tpv;
-        block_count += ch.steps;
-        L.chunk.push_back(ch);
-      }
-      ci.chunk_end = (int)L.chunk.size();
+    for (ColorInfo ci : P.color) {
+      ci.chunk_begin += nq;
+      ci.chunk_end += nq;
       L.color.push_back(ci);
     }
-    ei.nsolved = next;
-    for (int v : freev) new_local[v] = next++;
-    ei.nact = next;
-    for (int v : fixedv) new_local[v] = next++;
-    ei.ncolors = (int)L.color.size() - ei.cbase;
-    L.env.push_back(ei);
-    L.max_colors = std::max(L.max_colors, ei.ncolors);
-    L.max_env_vertices = std::max(L.max_env_vertices, vn);
-    for (int v = 0; v < vn; ++v) {
-      const int gnew = vo + new_local[v];
-      L.new_of_old[vo + v] = gnew;
-      const int k = off[v + 1] - off[v];
-      L.valence[gnew] = k;
-      double m = 0.0, hs = 0.0, logE = 0.0, rho = 0.0, nu = 0.0;
-      for (int s = off[v]; s < off[v + 1]; ++s) {
-        const int t = to + inc[s];
-        m += td.mass[t] / 4.0;
-        hs += std::cbrt(6.0 * td.vol[t]);
-        logE += std::log10(td.E[t]);
-        rho += td.rho[t];
-        nu += td.nu[t];
-      }
-      L.mass[gnew] = m;
-      // warm-start vertex constants: local length scale h (mean cube root of
-      // 6 V over the incident tets), log10(E / (rho h^2)), nu, valence / 20
-      float* w4 = &L.wstat[4 * (size_t)gnew];
-      if (k > 0) {
-        const double h = hs / k;
-        w4[0] = (float)h;
-        w4[1] = (float)(logE / k - std::log10(rho / k * h * h));
-        w4[2] = (float)(nu / k);
-        w4[3] = (float)(k / 20.0);
-      } else {
-        w4[0] = 1.0f;
-        w4[1] = w4[2] = w4[3] = 0.0f;
-      }
+    for (ChunkInfo ch : P.chunk) {
+      ch.block += nb;
+      L.chunk.push_back(ch);
     }
-    for (int c = ei.cbase; c < ei.cbase + ei.ncolors; ++c)
-      for (int q = L.color[c].chunk_begin; q < L.color[c].chunk_end; ++q)
-        L.chunk_owner.push_back(make_int2(c, e));
-    // slot records: (n0, n1, n2, record id) per slot, the record values in a
-    // table of this environment shared by every slot with the same values in
-    // the solver precision (record ids are environment-local, so a block can
-    // stage its environment's table in shared memory)
-    L.rec_idx.resize((size_t)block_count * 32, make_int4(0, 0, 0, 0));
-    RecordTable etab;
-    etab.fp64 = L.table.fp64;
-    std::vector<int> tet_rec(etab.fp64 ? tn : 0, -1);  // fp64: record of each tet
-    std::vector<std::pair<int, int4>> tlist;  // (owner, owner slot) per tet
-    std::vector<int> old_of_new_local(vn);
-    for (int v = 0; v < vn; ++v) old_of_new_local[new_local[v]] = v;
-    for (int ci_i = ei.cbase; ci_i < ei.cbase + ei.ncolors; ++ci_i) {
-      const ColorInfo ci = L.color[ci_i];
-      for (int q = ci.chunk_begin; q < ci.chunk_end; ++q) {
-        const ChunkInfo ch = L.chunk[q];
-        for (int lane = 0; lane < 32; ++lane) {
-          const int vi = lane / tpv, sub = lane % tpv;
-          const int gv = ci.vbegin + (q - ci.chunk_begin) * cpw + vi;
-          if (gv >= ci.vend) continue;
-          const int ov = old_of_new_local[gv - vo];
-          const int k = off[ov + 1] - off[ov];
-          for (int s = 0; s < ch.steps; ++s) {
-            const int j = s * tpv + sub;
-            if (j >= k) break;
-            const int t = to + inc[off[ov] + j];
-            const int a = loc[off[ov] + j];
-            const size_t blk = (size_t)ch.block + s;
-            int ids[3];
-            const double* bt = &td.b[(size_t)t * 12];
-            const double* pt = &td.p[(size_t)t * 3];
-            int n = 0, solved_in_tet = 0, owner = vn;
-            for (int qq = 0; qq < 4; ++qq) {
-              const int nl = new_local[tets[4 * (size_t)t + qq] - vo];
-              if (nl < ei.nsolved) {
-                ++solved_in_tet;
-                owner = std::min(owner, nl);
-              }
-              if (qq != a) ids[n++] = nl;
-            }
-            int rid;
-            if (etab.fp64) {
-              int& rec = tet_rec[t - to];
-              if (rec < 0) {
-                double val[12];
-                for (int i = 0; i < 3; ++i) {
-                  for (int c = 0; c < 3; ++c) val[4 * i + c] = bt[3 * i + c];
-                  val[4 * i + 3] = pt[i & 1];
-                }
-                rec = etab.insert(val);
-              }
-              rid = 4 * rec + a;
-            } else {
-              double val[12];
-              n = 0;
-              for (int qq = 0; qq < 4; ++qq) {
-                if (qq == a) continue;
-                for (int c = 0; c < 3; ++c) val[4 * n + c] = bt[qq * 3 + c];
-                val[4 * n + 3] = pt[n];
-                ++n;
-              }
-              // 4th value of the last row: this slot's share of the tet's
-              // strain energy
-              val[11] = 1.0 / solved_in_tet;
-              rid = etab.insert(val);
-            }
-            L.rec_idx[blk * 32 + lane] = make_int4(ids[0], ids[1], ids[2], rid);
-            if (owner == gv - vo) tlist.emplace_back(owner, make_int4(ids[0], ids[1], ids[2], rid));
-            L.n_slots++;
-          }
-        }
-      }
-    }
-    L.env.back().rbase = L.table.size();
-    L.env.back().nrec = etab.size();
-    // the tet list in owner order (neighbouring entries read nearby state)
-    std::stable_sort(tlist.begin(), tlist.end(),
-                     [](const std::pair<int, int4>& a, const std::pair<int, int4>& b) {
-                       return a.first < b.first;
-                     });
-    L.env.back().tbase = (int)L.tet_slot.size();
-    L.env.back().ntets = (int)tlist.size();
-    for (const auto& x : tlist) {
-      L.tet_owner.push_back(x.first);
-      L.tet_slot.push_back(x.second);
-    }
-    L.table.vals.insert(L.table.vals.end(), etab.vals.begin(), etab.vals.end());
-    L.max_env_records = std::max(L.max_env_records, etab.size());
+    for (int2 o : P.chunk_owner) L.chunk_owner.push_back(make_int2(o.x + nc, o.y));
+    L.rec_idx.insert(L.rec_idx.end(), P.rec_idx.begin(), P.rec_idx.end());
+    L.tet_slot.insert(L.tet_slot.end(), P.tet_slot.begin(), P.tet_slot.end());
+    L.tet_owner.insert(L.tet_owner.end(), P.tet_owner.begin(), P.tet_owner.end());
+    L.table.vals.insert(L.table.vals.end(), P.table.vals.begin(), P.table.vals.end());
+    L.max_valence = std::max(L.max_valence, P.max_valence);
+    L.max_colors = std::max(L.max_colors, P.max_colors);
+    L.max_env_vertices = std::max(L.max_env_vertices, P.max_env_vertices);
+    L.max_env_records = std::max(L.max_env_records, P.max_env_records);
+    L.n_slots += P.n_slots;
+    P = Layout();
   }
   return VBD_OK;
 }
@@ -1289,24 +1390,15 @@ void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, i
 }
 
 // Every environment in `parts` domains, appended to D; first[env] = its first
-// domain, smem[env] = the largest of its domains'.  The environments are
-// independent: host threads take them in turn.
+// domain, smem[env] = the largest of its domains'.
 void build_all_domains(const Layout& L, int ltpv, const double* X, int tpv, int parts,
                        bool sort_records, DomLayout& D, std::vector<int>& first,
                        std::vector<size_t>& smem) {
   const int n = (int)L.env.size();
   std::vector<DomLayout> each(n);
-  std::atomic<int> next{0};
-  auto work = [&]() {
-    for (int k; (k = next.fetch_add(1)) < n;)
-      build_domains(L, ltpv, X, k, tpv, parts, sort_records, each[k]);
-  };
-  const int nthreads =
-      std::min<int>(n, std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
-  std::vector<std::thread> pool;
-  for (int i = 1; i < nthreads; ++i) pool.emplace_back(work);
-  work();
-  for (auto& t : pool) t.join();
+  for_each_parallel(n, [&](int k) {
+    build_domains(L, ltpv, X, k, tpv, parts, sort_records, each[k]);
+  });
   first.resize(n);
   smem.assign(n, 0);
   for (int k = 0; k < n; ++k) {
@@ -1510,7 +1602,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   }
   s->tpv = tpv;
   s->L.table.fp64 = s->fp64;
-  rc = build_layout(X, V, tets, T, active, voff, toff, coloring, td, tpv,
+  rc = build_layout(V, tets, active, voff, toff, coloring, td, tpv,
                     (flags & VBD_ORDER_INDEX) != 0, s->L,
                     gpu_colors.empty() ? nullptr : gpu_colors.data());
   if (rc != VBD_OK) {
