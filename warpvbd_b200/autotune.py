@@ -7,9 +7,9 @@ and shape.  Measured on a B200 (per sweep, cantilever meshes):
   shared memory (block mode) wins;
 - at a few thousand, block mode wins only when the mesh is spread over a
   thread-block cluster;
-- beyond that, one cooperative launch with grid barriers (persistent mode)
-  or per-colour kernels in a graph (graph mode) is faster, and which lanes
-  per vertex are best changes again.
+- beyond that, one cooperative launch over all SMs (persistent mode; in fp64
+  from about a hundred vertices on) or per-colour kernels in a graph (graph
+  mode) is faster, and which lanes per vertex are best changes again.
 
 The autotuner measures instead of guessing.  For one mesh (or one batch of
 environments) it builds a solver per candidate launch shape, times a few
