@@ -505,6 +505,8 @@ def run_ours(args, envs, desc, batched):
     achieved = alg_bytes / (kernel_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peak()
     kernel = {"block": "env_step_kernel", "persist": "persist_kernel"}.get(mode, "color_kernel")
+    if args.precision == "fp64" and mode in ("block", "persist"):
+        kernel = "domain_kernel"
     prof = f"{args.workload}.{args.precision}" + (".warm" if warm is not None else "")
     tps = profile_traffic_per_slot(kernel, prof)
     traffic = None if tps is None else tps * float((iters * slots[None, :]).sum()) / args.steps
@@ -544,8 +546,8 @@ def run_ours(args, envs, desc, batched):
                                     "the positions in shared memory, DRAM traffic is a small "
                                     "fraction of the algorithmic bytes (ncu summary in "
                                     "profiles/)" if mode == "block" else
-                                    "latency: the per-colour dependency chain and grid "
-                                    "barriers (ncu summary in profiles/)",
+                                    "latency: the per-colour dependency chain and the "
+                                    "handoff between blocks (ncu summary in profiles/)",
                          "kernel_ms_per_step": kernel_ms / args.steps},
             "e2e": {"value": e2e, "unit": "sim-s/wall-s",
                     "h2d_bytes_per_step": 24 * n_vertices,

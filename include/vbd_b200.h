@@ -88,9 +88,9 @@ typedef struct vbd_solver vbd_solver;
  * would otherwise set the step time; the planner uses it only when its
  * duration model says it shortens the step */
 #define VBD_TIERED_WIDE 0x80
-/* persistent mode: separate the colours of a sweep with grid barriers instead
- * of the default neighbour-scoped readiness (each block waits only for the
- * blocks owning vertices that share a tet with its own) */
+/* persistent mode: separate the colours of a sweep with grid-wide barriers
+ * instead of the default neighbour-scoped readiness (each block waits only for
+ * the vertices, or the blocks owning vertices, that share a tet with its own) */
 #define VBD_PERSIST_GRID_BARRIERS 0x8000
 /* block mode: thread blocks per cluster (1 to 16; 0 = automatic).  An
  * environment much heavier than the others is split over all blocks of one
@@ -153,7 +153,7 @@ int vbd_create_batched(const double* rest_positions, int n_vertices, const int32
 void vbd_destroy(vbd_solver* s);
 
 /* No counterpart in the reference.  Bounds every device-side wait of the
- * persistent mode (VBD_MODE_PERSIST grid barriers): a wait gives up after
+ * persistent mode, and in fp64 of the block mode's clusters: a wait gives up after
  * max_polls polls or max_wait_ns nanoseconds, whichever comes first, and the
  * step then fails with VBD_ERR_TIMEOUT (positions undefined until
  * vbd_reset / vbd_set_positions).  Defaults: 2^26 polls, 2 s. */
