@@ -5,7 +5,7 @@ not fit in shared memory against the per-colour graph mode."""
 import numpy as np
 import pytest
 
-from warpvbd_b200 import VBDSolver, _lib, scenes
+from warpvbd_b200 import BatchedVBDSolver, VBDSolver, _lib, scenes
 from oracle.oracle import OracleSolver
 
 pytestmark = pytest.mark.gpu
@@ -106,3 +106,40 @@ def test_meshes_whose_domains_do_not_fit_match_graph_mode():
         y = g.step(g.old_positions, 1e-3).numpy()
         assert p.last_iterations == g.last_iterations
         assert np.abs(x - y).max() < 1e-13 * diag
+
+
+def _steps(solver, n=3):
+    out = [np.array(solver.step(1e-3)) for _ in range(n)]
+    return out, np.array(solver.positions())
+
+
+@pytest.mark.parametrize("threads", [64, 128, 256])
+def test_environments_that_fill_an_sm_take_the_same_steps_at_any_thread_count(threads):
+    """A block whose shared memory leaves no room for another takes 512 threads whatever was
+    asked for; small environments beside it and without it take what was asked."""
+    large, small = scenes.mass_spring(15, 30), scenes.mass_spring(3, 4)
+    for envs in ([large, small], [small, small]):
+        runs = []
+        for th in (512, threads):
+            sol = BatchedVBDSolver(envs, dx_tol=1e-7, max_iter=1000, tiered=True, cluster=2, tpv=4,
+                                   block_threads=th)
+            runs.append(_steps(sol))
+            sol.close()
+        assert all((a == b).all() for a, b in zip(runs[0][0], runs[1][0]))
+        assert (runs[0][1] == runs[1][1]).all()
+
+
+def test_environments_set_up_together_are_those_set_up_alone():
+    """The setup builds the environments of a batch on several host threads."""
+    envs = [scenes.mass_spring(2 + k % 4, 2 + k % 3) for k in range(21)]
+    shape = dict(dx_tol=1e-7, max_iter=1000, cluster=1, tpv=4, block_threads=128)
+    sol = BatchedVBDSolver(envs, **shape)
+    its, x = _steps(sol)
+    sol.close()
+    at = np.cumsum([0] + [e.n_vertices for e in envs])
+    for k, e in enumerate(envs):
+        sol = BatchedVBDSolver([e], **shape)
+        its1, x1 = _steps(sol)
+        sol.close()
+        assert [int(i[0]) for i in its1] == [int(i[k]) for i in its]
+        assert (x1 == x[at[k]:at[k + 1]]).all()
