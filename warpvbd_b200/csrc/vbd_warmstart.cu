@@ -247,8 +247,11 @@ __global__ void __launch_bounds__(kFwdThreads, 4) mlp_forward_kernel(const float
   extern __shared__ __align__(16) float fw[];
   constexpr int TILE = 16 * SPT, SP = SPT / 2;
   const int t = threadIdx.x, tx = t & 7, ty = t >> 3;
+  // all of a thread's weights in flight at once: 1 to 2 us of a launch
+#pragma unroll
   for (int i = t; i < kWsIn * kWsHidden; i += kFwdThreads)
     fw[kFwW1T + i] = P[kWsW1 + i % kWsHidden * kWsIn + i / kWsHidden];
+#pragma unroll 16
   for (int i = t; i < kWsHidden * kWsHidden; i += kFwdThreads)
     fw[kFwW2T + i] = P[kWsW2 + i % kWsHidden * kWsHidden + i / kWsHidden];
   for (int i = t; i < kWsHidden; i += kFwdThreads) {
