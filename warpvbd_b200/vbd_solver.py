@@ -163,7 +163,8 @@ class VBDSolver:
                  steps and 9.6e-5 on the 256-environment batch) or "fp32"
                  (everything fp32)
       mode       "auto", "block", "graph", "hostloop" or "persist" (see include/vbd_b200.h)
-      tpv, block_threads   launch shape (0 = automatic)
+      tpv, block_threads   launch shape (0 = automatic; in fp64 the persistent mode
+                 takes its own thread count)
       cluster    block mode: spread the mesh over this many thread blocks of one
                  cluster (1 to 16; 0 = automatic)
       order_index  keep ascending vertex index inside a colour (default: by valence)
