@@ -6,6 +6,7 @@
 #include <math.h>
 
 #include "vbd_internal.h"
+#include "vbd_solve.h"
 
 namespace vbd {
 
@@ -450,24 +451,7 @@ __device__ __forceinline__ bool chol_solve3(const Real* h, const Real* g, Real* 
   return (h[0] > Real(0)) && (d1 > Real(0)) && (d2 > Real(0));
 }
 
-// The same step in fp64 by cofactors: H^-1 = adj(H) / det(H), one reciprocal
-// where the Cholesky form chains three square roots and three divides, which
-// one lane per vertex runs while the warp waits.  H is positive definite when
-// its leading minors are positive.  Determinants near the ends of the double
-// range take the Cholesky form.
-__device__ __forceinline__ bool solve3(const double* h, const double* g, double* x) {
-  const double c00 = cross2(h[3], h[5], h[4], h[4]), c01 = cross2(h[2], h[4], h[1], h[5]),
-               c02 = cross2(h[1], h[4], h[2], h[3]), c11 = cross2(h[0], h[5], h[2], h[2]),
-               c12 = cross2(h[1], h[2], h[0], h[4]), c22 = cross2(h[0], h[3], h[1], h[1]);
-  const double det = dot3(h[0], c00, h[1], c01, h[2], c02);
-  if (!(fabs(det) > 1e-250 && fabs(det) < 1e250)) return chol_solve3<double>(h, g, x);
-  const double r = -reciprocal64(det);
-  // products the caller adds to: kept from being fused into those additions
-  x[0] = __dmul_rn(dot3(c00, g[0], c01, g[1], c02, g[2]), r);
-  x[1] = __dmul_rn(dot3(c01, g[0], c11, g[1], c12, g[2]), r);
-  x[2] = __dmul_rn(dot3(c02, g[0], c12, g[1], c22, g[2]), r);
-  return (h[0] > 0.0) && (c22 > 0.0) && (det > 0.0);
-}
+// fp64: vbd_solve.h
 __device__ __forceinline__ bool solve3(const float* h, const float* g, float* x) {
   return chol_solve3<float>(h, g, x);
 }
