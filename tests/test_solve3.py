@@ -1,5 +1,5 @@
-"""The fp64 3x3 solve of the vertex update (warpvbd_b200/csrc/vbd_solve.h), compiled for the
-host, against exact rational arithmetic: blocks of well-shaped tets, of nearly incompressible
+"""The fp64 3x3 solve and the reciprocal of the vertex update (warpvbd_b200/csrc/vbd_solve.h),
+compiled for the host, against exact rational arithmetic: blocks of well-shaped tets, of nearly incompressible
 ones (one stiff direction, lambda / mu up to 1e12) and of very different scales."""
 import ctypes
 import os
@@ -14,15 +14,22 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 
 
 @pytest.fixture(scope="module")
-def solve3(tmp_path_factory):
+def library(tmp_path_factory):
     d = tmp_path_factory.mktemp("solve3")
     src, so = d / "solve3.cpp", d / "solve3.so"
     src.write_text('#include "vbd_solve.h"\n'
                    'extern "C" int solve(const double* h, const double* g, double* x) {\n'
-                   '  return vbd::solve3(h, g, x);\n}\n')
+                   '  return vbd::solve3(h, g, x);\n}\n'
+                   'extern "C" double newton(double x, double y) {\n'
+                   '  return vbd::newton_reciprocal(x, y);\n}\n')
     subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared",
                     f"-I{CSRC}", str(src), "-o", str(so)], check=True)
-    f = ctypes.CDLL(str(so)).solve
+    return ctypes.CDLL(str(so))
+
+
+@pytest.fixture(scope="module")
+def solve3(library):
+    f = library.solve
     f.argtypes = [ctypes.POINTER(ctypes.c_double)] * 3
 
     def run(h, g):
@@ -80,3 +87,19 @@ def test_error_grows_with_the_condition_number_only(solve3, k, scale):
     np.full((3, 3), np.nan), np.diag([1.0, np.nan, 1.0]), -np.eye(3)])
 def test_blocks_that_are_not_positive_definite_are_reported(solve3, H):
     assert not solve3(_packed(H), np.ones(3))[0]
+
+
+@pytest.mark.parametrize("start", [-2.0 ** -20, -2.0 ** -24, 0.0, 2.0 ** -27, 2.0 ** -20])
+def test_newton_reciprocal_is_rounded_once(library, start):
+    """From an approximation with relative error e <= 2^-20 the first step leaves e^2 = 2^-40
+    and two roundings, the second (2^-40 + 2^-52)^2 and one rounding of a term of that size:
+    half a unit in the last place of the result, plus less than 2^-79 of it."""
+    f = library.newton
+    f.argtypes, f.restype = [ctypes.c_double, ctypes.c_double], ctypes.c_double
+    rng = np.random.default_rng(7)
+    for x in np.concatenate([1.0 + rng.random(400), 4.0 + rng.random(400) * 1e-6,
+                             10.0 ** rng.uniform(0, 300, 400)]):
+        y = f(x, (1.0 / x) * (1.0 + start))
+        exact = 1 / Fraction(float(x))
+        assert abs(Fraction(y) - exact) <= (Fraction(float(np.spacing(y))) / 2
+                                            + exact / 2 ** 79)

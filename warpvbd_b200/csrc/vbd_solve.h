@@ -1,5 +1,5 @@
-// The fp64 3x3 solve of a vertex's Newton step.  Plain C++ apart from one
-// rounding intrinsic, so that it also compiles for the host.
+// The fp64 3x3 solve of a vertex's Newton step, and the reciprocal of its slots.  Plain C++
+// apart from one rounding intrinsic, so that it also compiles for the host.
 #pragma once
 #include <cmath>
 
@@ -18,6 +18,14 @@ VBD_HOST_DEVICE double mul_rounded(double a, double b) {
 #else
   return a * b;
 #endif
+}
+
+// 1 / x from an approximation y of 20 correct bits or more (rcp.approx.ftz.f64's): two Newton
+// steps y (2 - x y), each of which squares the relative error.  The second adds less than
+// 2^-79 / x to the rounding of the result.
+VBD_HOST_DEVICE double newton_reciprocal(double x, double y) {
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
 }
 
 // Solves H x = -g (h = h00 h01 h02 h11 h12 h22) by H = L D L^T; false when a pivot is not
