@@ -143,3 +143,26 @@ def test_environments_set_up_together_are_those_set_up_alone():
         sol.close()
         assert [int(i[0]) for i in its1] == [int(i[k]) for i in its]
         assert (x1 == x[at[k]:at[k + 1]]).all()
+
+
+@pytest.mark.parametrize("polls", [0, 1, 3, 10, 30, 100, 300])
+def test_a_step_in_which_a_wait_expired_never_passes_as_finished(polls):
+    """With short limits some blocks of a one-sweep step give up, some before the block that
+    clears the status has started: the step either reports it or has the whole result."""
+    s = scenes.cantilever(40)
+    kw = dict(s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1, mode="persist")
+    p, q = VBDSolver(**kw), VBDSolver(**kw)
+    ref = q.step(q.old_positions, 1e-3).numpy()
+    L = _lib.load()
+    assert L.vbd_set_wait_limits(p._h, polls, 2_000_000_000) == 0
+    for _ in range(40):
+        p.reset()
+        try:
+            x = p.step(p.old_positions, 1e-3).numpy()
+        except _lib.VBDError as e:
+            assert e.status == _lib.ERR_TIMEOUT
+        else:
+            assert np.array_equal(x, ref)
+    assert L.vbd_set_wait_limits(p._h, 1 << 26, 2_000_000_000) == 0
+    p.reset()
+    assert np.array_equal(p.step(p.old_positions, 1e-3).numpy(), ref)

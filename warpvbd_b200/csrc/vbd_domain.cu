@@ -30,7 +30,8 @@
 //
 // Every wait is bounded (polls and wall clock); on expiry the block writes the
 // step's number to the abort word, sets the timeout status and returns, and the
-// others leave at their next wait.  The blocks of one environment are resident
+// others leave at their next wait.  The host takes a step whose abort word changed as
+// timed out, whatever the status words hold.  The blocks of one environment are resident
 // together: they form one cluster, or the launch is cooperative.
 //
 // What bounds it: up to a few thousand vertices the chain of one colour -- one
@@ -334,8 +335,8 @@ __global__ void __launch_bounds__(kDomMaxThreads)
   }
   for (int i = tid; i < ncolors; i += nt) s_color[i] = d.color[di.cbase + i];
   if (tid < 2) s_stat[tid] = 0u;
-  // only ORed from here on; the other blocks can do that only after this
-  // block's first post
+  // ORed from here on.  Another block whose wait expires before this store loses its
+  // bit; the abort word, which it sets too, tells the host
   if (tid == 0 && di.rank == 0) m.status[di.env] = 0u;
   __syncthreads();
   const unsigned long long seq = (unsigned long long)d.seq << 28;  // tags: step, sweep / exchange

@@ -620,7 +620,7 @@ struct vbd_solver {
   DevBuf<unsigned char> d_rec_tab;
   int fmt = kFmtIdx32;
   DevBuf<int> d_valence, d_map, d_iters;
-  DevBuf<unsigned> d_status;
+  DevBuf<unsigned> d_status;  // per env, then the word of expired waits (DomDev::abort)
   // per env: largest |dx| component of the last allowed sweep (DevMesh::dxmax)
   DevBuf<unsigned long long> d_dxmax;
   unsigned long long* h_dxmax = nullptr;  // pinned
@@ -652,7 +652,7 @@ struct vbd_solver {
   DevBuf<int4> d_dom_tet;
   DevBuf<int> d_dom_tet_owner;
   DevBuf<ulonglong2> d_dom_mail, d_dom_post;
-  DevBuf<unsigned> d_dom_abort;
+  unsigned dom_abort_seen = 0;  // the abort word when the last step was finished
   PersistLimits wait_limits{1ll << 26, 2000000000ull};  // every grid-barrier wait
   // block-mode work map: (environment, rank, group size) per thread block
   int cluster = 1;           // blocks per cluster = group size of a split environment
@@ -829,7 +829,6 @@ void free_solver(vbd_solver* s) {
   s->d_nbr_idx.release();
   s->d_epoch.release();
   for (auto& f : s->d_dom_first) f.release();
-  s->d_dom_abort.release();
   s->d_dom.release();
   s->d_dom_color.release();
   s->d_dom_chunk.release();
@@ -1423,7 +1422,7 @@ DomDev dom_dev(const vbd_solver* s) {
   d.tet_owner = s->d_dom_tet_owner.p;
   d.mail = s->d_dom_mail.p;
   d.post = s->d_dom_post.p;
-  d.abort = s->d_dom_abort.p;
+  d.abort = s->d_status.p + s->n_env;
   d.seq = s->dom_seq;
   d.grid_sync = (s->flags & VBD_PERSIST_GRID_BARRIERS) ? 1 : 0;
   return d;
@@ -1704,7 +1703,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   if (!err && bad(s->d_io.alloc(3 * (size_t)V), "io")) err = 1;
   if (!err && bad(s->d_tol.alloc(s->n_env), "tol")) err = 1;
   if (!err && bad(s->d_iters.alloc(s->n_env), "iters")) err = 1;
-  if (!err && bad(s->d_status.alloc(s->n_env), "status")) err = 1;
+  if (!err && bad(s->d_status.alloc(s->n_env + 1), "status")) err = 1;
   if (!err && bad(s->d_dxmax.alloc(s->n_env), "dxmax")) err = 1;
   if (!err && bad(s->d_params.alloc(1), "params")) err = 1;
   if (!err && bad(s->d_ctl.alloc(1), "ctl")) err = 1;
@@ -1769,12 +1768,10 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
           bad(s->d_dom_tet_owner.upload(D.tet_owner, st), "domains") ||
           bad(s->d_dom_mail.alloc(split ? 3 * (size_t)V : 1), "domains") ||
           bad(s->d_dom_post.alloc((size_t)posts), "domains") ||
-          bad(s->d_dom_abort.alloc(1), "domains") ||
           bad(cudaMemsetAsync(s->d_dom_mail.p, 0, sizeof(ulonglong2) * s->d_dom_mail.n, st),
               "domains") ||
           bad(cudaMemsetAsync(s->d_dom_post.p, 0, sizeof(ulonglong2) * s->d_dom_post.n, st),
-              "domains") ||
-          bad(cudaMemsetAsync(s->d_dom_abort.p, 0, sizeof(unsigned), st), "domains"))
+              "domains"))
         err = 1;
       cudaStreamSynchronize(st);  // D and first go out of scope
       if (block_mode) {
@@ -1842,14 +1839,15 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
       cudaStreamSynchronize(st);
     }
     cudaMemsetAsync(s->d_iters.p, 0, sizeof(int) * s->n_env, st);
-    cudaMemsetAsync(s->d_status.p, 0, sizeof(unsigned) * s->n_env, st);
+    cudaMemsetAsync(s->d_status.p, 0, sizeof(unsigned) * (s->n_env + 1), st);
     cudaMemsetAsync(s->d_dxmax.p, 0, sizeof(unsigned long long) * s->n_env, st);
   }
   if (!err && bad(cudaMallocHost(reinterpret_cast<void**>(&s->h_iters), sizeof(int) * s->n_env),
                   "pinned"))
     err = 1;
   if (!err &&
-      bad(cudaMallocHost(reinterpret_cast<void**>(&s->h_status), sizeof(unsigned) * s->n_env),
+      bad(cudaMallocHost(reinterpret_cast<void**>(&s->h_status),
+                         sizeof(unsigned) * (s->n_env + 1)),
           "pinned"))
     err = 1;
   if (!err && bad(cudaMallocHost(reinterpret_cast<void**>(&s->h_dxmax),
@@ -2159,13 +2157,20 @@ int finish(vbd_solver* s, int* iters_out, bool warm_step) {
   cudaStream_t st = s->stream;
   CUDA_TRY(cudaMemcpyAsync(s->h_iters, s->d_iters.p, sizeof(int) * s->n_env,
                            cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaMemcpyAsync(s->h_status, s->d_status.p, sizeof(unsigned) * s->n_env,
+  CUDA_TRY(cudaMemcpyAsync(s->h_status, s->d_status.p, sizeof(unsigned) * (s->n_env + 1),
                            cudaMemcpyDeviceToHost, st));
   if (warm_step && s->h_ws_err)
     CUDA_TRY(cudaMemcpyAsync(s->h_ws_err, s->d_ws_err.p, sizeof(unsigned),
                              cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   s->pending = false;
+  // a wait expired in a step since the last one finished: an environment's own bit may be
+  // lost (its first block clears the word when it starts, which may be after another block
+  // of it gave up), so none of its results is taken
+  if (s->h_status[s->n_env] != s->dom_abort_seen) {
+    s->dom_abort_seen = s->h_status[s->n_env];
+    for (int e = 0; e < s->n_env; ++e) s->h_status[e] |= kStatTimeout;
+  }
   if (cudaEventElapsedTime(&s->kernel_ms_last, s->ev_k0, s->ev_k1) != cudaSuccess) {
     s->kernel_ms_last = -1.f;
     cudaGetLastError();  // not a step failure: keep it out of the next launch check
@@ -2176,10 +2181,11 @@ int finish(vbd_solver* s, int* iters_out, bool warm_step) {
                          : 2 + s->h_iters[0] * ((int)s->L.color.size() + 1);
   if (iters_out) std::memcpy(iters_out, s->h_iters, sizeof(int) * s->n_env);
   // environments that used every allowed sweep recorded the largest |dx|
-  // component of the last one: read it, then clear the words for the next
-  // step that reaches its cap (the stream is idle here)
+  // component of the last one (some vertices of a timed-out one may have): read it, then
+  // clear the words for the next step that reaches its cap (the stream is idle here)
   bool capped = false;
-  for (int e = 0; e < s->n_env; ++e) capped |= (s->h_status[e] & kStatIterCap) != 0;
+  for (int e = 0; e < s->n_env; ++e)
+    capped |= (s->h_status[e] & (kStatIterCap | kStatTimeout)) != 0;
   std::fill(s->final_dx.begin(), s->final_dx.end(), std::nan(""));
   if (capped) {
     CUDA_TRY(cudaMemcpy(s->h_dxmax, s->d_dxmax.p, sizeof(unsigned long long) * s->n_env,
