@@ -166,3 +166,44 @@ def test_a_step_in_which_a_wait_expired_never_passes_as_finished(polls):
     assert L.vbd_set_wait_limits(p._h, 1 << 26, 2_000_000_000) == 0
     p.reset()
     assert np.array_equal(p.step(p.old_positions, 1e-3).numpy(), ref)
+
+
+def test_automatic_mode_takes_the_calls_of_block_mode():
+    """A mesh that block mode holds, stepped over the whole device by the automatic mode:
+    tolerances per environment, the timeline and the direct write of positions."""
+    import ctypes
+    import torch
+    s = scenes.cantilever(40)
+    kw = dict(s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1000)
+    a, b = VBDSolver(**kw), VBDSolver(**kw)
+    assert a.info()["mode"] == 0x400
+    L = _lib.load()
+    it = np.zeros(1, np.int32)
+    out = torch.empty(s.vertices.shape, dtype=torch.float64).pin_memory().numpy()
+    _lib.check(L.vbd_set_trace(a._h, 1))
+    for tol in (1e-4, 1e-7):
+        x = b.step(b.old_positions, 1e-3, dx_tol=tol).numpy()
+        st = L.vbd_step_batched_to(a._h, 1e-3, 1.0, _lib.ptr(np.array([tol]), "d"), 1000,
+                                   it.ctypes.data_as(ctypes.POINTER(ctypes.c_int)),
+                                   _lib.ptr(out, "d"))
+        assert st == _lib.OK
+        assert it[0] == b.last_iterations
+        assert np.array_equal(out, x)
+    n = ctypes.c_int(0)
+    _lib.check(L.vbd_get_trace(a._h, None, 0, ctypes.byref(n)))
+    rec = np.zeros((n.value, 4), np.uint64)
+    _lib.check(L.vbd_get_trace(a._h, rec.ctypes.data_as(ctypes.POINTER(ctypes.c_ulonglong)),
+                               n.value, ctypes.byref(n)))
+    assert n.value == a.info()["n_blocks"]
+    assert (rec[:, 1] > rec[:, 0]).all() and (rec[:, 3] >> np.uint64(8) == it[0]).all()
+    # refused before, refused now: the same call in persistent mode by name
+    c = VBDSolver(**kw, mode="persist")
+    st = L.vbd_step_batched(c._h, 1e-3, 1e-7, _lib.ptr(np.array([1e-7]), "d"), 1000,
+                            it.ctypes.data_as(ctypes.POINTER(ctypes.c_int)))
+    assert st == _lib.ERR_UNSUPPORTED
+
+
+def test_automatic_mode_keeps_a_cluster_size_asked_for():
+    s = scenes.cantilever(40)
+    sol = VBDSolver(**s.solver_kwargs(), damping_coefficient=0.0, cluster=4)
+    assert sol.info()["mode"] == 0x100 and sol.info()["cluster"] == 4

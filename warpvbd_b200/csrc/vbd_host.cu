@@ -639,6 +639,10 @@ struct vbd_solver {
   // fp64 by domains (vbd_domain.cu): layouts of 1, `cluster` and `cluster_wide`
   // domains per environment (block mode), or one of ndom (persistent mode)
   bool by_domains = false;
+  // automatic mode took the persistent step for a mesh that block mode would hold: calls
+  // that need block mode (tolerances per environment, the timeline, the direct write of
+  // positions) are taken as there
+  bool block_calls = false;
   int ndom = 0, dom_tpv = 0;
   unsigned dom_seq = 0;
   std::vector<size_t> dom_smem[3];  // per environment
@@ -1510,7 +1514,9 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     }
   }
   // mode / threads / tpv
+  const int tpv_arg = tpv, threads_arg = threads;
   const bool tpv_given = tpv != 0;
+  const int cl = (flags >> VBD_CLUSTER_SHIFT) & 0x1F;
   int mode = flags & VBD_MODE_MASK;
   // provisional environment size bound for the shared-memory check
   int max_env_v = 0;
@@ -1526,10 +1532,13 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     // persistent step by domains wins from a few dozen vertices on (us per sweep,
     // one block or cluster -> domains: 189 vertices 18.9 -> 13.7, 1,025 vertices
     // 41 -> 15, 1,808 vertices 44 -> 19).
-    if (s->n_env > 1)
+    // A cluster size asked for is block mode's.
+    const bool holds = fits && V <= 2048;
+    if (s->n_env > 1 || (holds && (!s->fp64 || V <= 96 || cl)))
       mode = VBD_MODE_BLOCK;
     else
-      mode = (fits && V <= (s->fp64 ? 96 : 2048)) ? VBD_MODE_BLOCK : VBD_MODE_PERSIST;
+      mode = VBD_MODE_PERSIST;
+    s->block_calls = holds && mode == VBD_MODE_PERSIST;
   }
   if (mode == VBD_MODE_BLOCK && !fits) {
     delete s;
@@ -1547,7 +1556,6 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   }
   s->mode = mode;
   const bool block_mode = mode == VBD_MODE_BLOCK;
-  const int cl = (flags >> VBD_CLUSTER_SHIFT) & 0x1F;
   // the cluster field is 5 bits wide and nothing lies above it: a set bit
   // there is a cluster size that did not fit (or a negative one)
   if (cl > 16 || (static_cast<unsigned>(flags) >> (VBD_CLUSTER_SHIFT + 5)) != 0u) {
@@ -1783,6 +1791,11 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
       }
     }
   }
+  if (!err && s->block_calls && !s->by_domains) {  // as without domains
+    free_solver(s);
+    return create_impl(X, V, tets, T, rho, E, nu, active, kd, gravity, coloring, voff, toff,
+                       flags | VBD_MODE_BLOCK, tpv_arg, threads_arg, device, out);
+  }
   if (!err && mode == VBD_MODE_PERSIST && !s->by_domains) {
     // resident blocks, but no more than the largest colour can keep busy
     // (one chunk per warp): fewer blocks make cheaper grid barriers
@@ -1946,7 +1959,7 @@ int set_params(vbd_solver* s, double dt, double tol, int max_iter) {
   p.strict_spd = (s->flags & VBD_STRICT_SPD) ? 1 : 0;
   p.warm = s->warm ? 1 : 0;
   p.tab_in_smem = s->tab_in_smem ? 1 : 0;
-  p.trace = (s->trace_on && s->mode == VBD_MODE_BLOCK) ? s->d_trace.p : nullptr;
+  p.trace = s->trace_on && (s->mode == VBD_MODE_BLOCK || s->block_calls) ? s->d_trace.p : nullptr;
   if (s->params_valid && std::memcmp(&p, &s->cur_params, sizeof p) == 0) return VBD_OK;
   // the pinned staging struct may still be read by an earlier copy
   CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -2017,16 +2030,15 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
   cudaStream_t st = s->stream;
   int launches = 0;
   if (s->by_domains) s->dom_seq = s->dom_seq + 1 < (1u << 28) ? s->dom_seq + 1 : 1;
+  const double* dtol = nullptr;
+  if (tol_env) {  // block mode, or a solver that takes its calls
+    CUDA_TRY(cudaStreamSynchronize(st));
+    CUDA_TRY(cudaMemcpy(s->d_tol.p, tol_env, sizeof(double) * s->n_env, cudaMemcpyHostToDevice));
+    dtol = s->d_tol.p;
+  }
+  if (s->cur_params.trace)
+    CUDA_TRY(cudaMemsetAsync(s->d_trace.p, 0, sizeof(unsigned long long) * s->d_trace.n, st));
   if (s->mode == VBD_MODE_BLOCK) {
-    const double* dtol = nullptr;
-    if (tol_env) {
-      CUDA_TRY(cudaStreamSynchronize(st));
-      CUDA_TRY(cudaMemcpy(s->d_tol.p, tol_env, sizeof(double) * s->n_env,
-                          cudaMemcpyHostToDevice));
-      dtol = s->d_tol.p;
-    }
-    if (s->cur_params.trace)
-      CUDA_TRY(cudaMemsetAsync(s->d_trace.p, 0, sizeof(unsigned long long) * s->d_trace.n, st));
     if (s->warm) {
       NvtxRange nw("vbd_warm_start");
       // features of the coming step, then the network's predicted corrections
@@ -2096,7 +2108,7 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
     ++launches;
     if (s->by_domains) {
       CUDA_TRY(launch_domain(s->material, s->dom_tpv, s->threads, m, s->cur_params, dom_dev(s),
-                             nullptr, s->wait_limits, s->ndom, 1, true, s->dom_smem[0][0], st));
+                             dtol, s->wait_limits, s->ndom, 1, true, s->dom_smem[0][0], st));
     } else {
       PersistNbr nbr{};
       if (s->persist_scoped) nbr = PersistNbr{s->d_nbr_off.p, s->d_nbr_idx.p, s->d_epoch.p};
@@ -2132,9 +2144,11 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
   }
   CUDA_TRY(cudaEventRecord(s->ev_k1, st));
   s->launches_pending = launches;
-  s->trace_pending = s->cur_params.trace && s->mode == VBD_MODE_BLOCK
-                         ? (int)(s->work.size() + s->work2.size() + s->work3.size())
-                         : 0;
+  s->trace_pending = 0;
+  if (s->cur_params.trace)
+    s->trace_pending = s->mode == VBD_MODE_BLOCK
+                           ? (int)(s->work.size() + s->work2.size() + s->work3.size())
+                           : s->ndom;
   s->pending = true;
   s->ws_history = true;  // ut now holds this step's inertia target
   return VBD_OK;
@@ -2347,7 +2361,7 @@ int vbd_set_trace(vbd_solver* s, int enable) {
   DeviceGuard dg(s->device);
   if (enable && !s->d_trace.p) {
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    CUDA_TRY(s->d_trace.alloc(4 * (s->d_work.n + s->d_work2.n + s->d_work3.n)));
+    CUDA_TRY(s->d_trace.alloc(4 * (s->d_work.n + s->d_work2.n + s->d_work3.n + s->ndom)));
     CUDA_TRY(cudaMemset(s->d_trace.p, 0, sizeof(unsigned long long) * s->d_trace.n));
   }
   s->trace_on = enable != 0;
@@ -2399,7 +2413,7 @@ int vbd_step_batched(vbd_solver* s, double dt, double tol, const double* tol_per
   if (!s) return fail(VBD_ERR_INVALID_ARG, "NULL solver");
   NvtxRange nr("vbd_step");
   DeviceGuard dg(s->device);
-  if (tol_per_env && s->mode != VBD_MODE_BLOCK)
+  if (tol_per_env && s->mode != VBD_MODE_BLOCK && !s->block_calls)
     return fail(VBD_ERR_UNSUPPORTED, "per-environment tolerances need block mode");
   int rc = enqueue_step(s, dt, tol, tol_per_env, max_iter);
   if (rc != VBD_OK) return rc;
@@ -2414,10 +2428,10 @@ int vbd_step_batched_to(vbd_solver* s, double dt, double tol, const double* tol_
   if (!s || !iterations_out || !positions_out) return fail(VBD_ERR_INVALID_ARG, "NULL argument");
   NvtxRange nr("vbd_step");
   DeviceGuard dg(s->device);
-  if (tol_per_env && s->mode != VBD_MODE_BLOCK)
+  if (tol_per_env && s->mode != VBD_MODE_BLOCK && !s->block_calls)
     return fail(VBD_ERR_UNSUPPORTED, "per-environment tolerances need block mode");
   double* dptr = nullptr;
-  if (s->mode == VBD_MODE_BLOCK &&
+  if ((s->mode == VBD_MODE_BLOCK || s->block_calls) &&
       cudaHostGetDevicePointer(reinterpret_cast<void**>(&dptr), positions_out, 0) != cudaSuccess) {
     cudaGetLastError();  // not page-locked and mapped: copy after the step instead
     dptr = nullptr;
