@@ -504,9 +504,7 @@ def run_ours(args, envs, desc, batched):
     kernel_ms = float(np.sum(detail["kernel_ms"]))
     achieved = alg_bytes / (kernel_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peak()
-    kernel = {"block": "env_step_kernel", "persist": "persist_kernel"}.get(mode, "color_kernel")
-    if args.precision == "fp64" and mode in ("block", "persist"):
-        kernel = "domain_kernel"
+    kernel = info["kernel"]
     prof = f"{args.workload}.{args.precision}" + (".warm" if warm is not None else "")
     tps = profile_traffic_per_slot(kernel, prof)
     traffic = None if tps is None else tps * float((iters * slots[None, :]).sum()) / args.steps

@@ -238,6 +238,11 @@ typedef struct vbd_info_t {
                                  warm-start feature and inference kernels */
 } vbd_info_t;
 int vbd_get_info(vbd_solver* s, vbd_info_t* info);
+/* Name of the kernel that runs the solver's sweeps: "domain_kernel" (fp64, block and
+ * persistent mode, when a domain of every environment fits in a block's shared memory),
+ * "env_step_kernel" (block mode otherwise), "persist_kernel" (persistent mode otherwise) or
+ * "color_kernel" (graph and host-loop mode). */
+const char* vbd_step_kernel(vbd_solver* s);
 
 /* The CUDA stream (cudaStream_t) all of the solver's work is enqueued on. */
 void* vbd_get_stream(vbd_solver* s);

@@ -118,6 +118,7 @@ SIGNATURES = {
     "vbd_set_velocities": (ctypes.c_int, [_vp, _d]),
     "vbd_get_color_groups": (ctypes.c_int, [_vp, _i, _ip, _ip]),
     "vbd_get_info": (ctypes.c_int, [_vp, ctypes.POINTER(VBDInfo)]),
+    "vbd_step_kernel": (ctypes.c_char_p, [_vp]),
     "vbd_get_stream": (_vp, [_vp]),
     "vbd_step_noalloc": (ctypes.c_int, [_vp, ctypes.c_double, ctypes.c_double, ctypes.c_int,
                                         _ip]),
@@ -179,6 +180,15 @@ def check(status, what=""):
         text = L.vbd_status_string(status).decode()
         raise VBDError(status, f"{what}: {text}: {msg}".strip(": "))
     return status
+
+
+def info(handle):
+    """The solver's vbd_info_t as a dict, and the name of its step kernel."""
+    L = load()
+    inf = VBDInfo()
+    check(L.vbd_get_info(handle, ctypes.byref(inf)))
+    return dict({n: getattr(inf, n) for n, _ in VBDInfo._fields_},
+                kernel=L.vbd_step_kernel(handle).decode())
 
 
 def ptr(a, kind):

@@ -100,9 +100,7 @@ class BatchedVBDSolver:
         self.last_status = _lib.OK
 
     def info(self):
-        inf = _lib.VBDInfo()
-        _lib.check(_lib.load().vbd_get_info(self._h, ctypes.byref(inf)))
-        return {n: getattr(inf, n) for n, _ in _lib.VBDInfo._fields_}
+        return _lib.info(self._h)
 
     @property
     def stream(self):

@@ -1567,14 +1567,17 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   // 9.0, 16 environments 8.5 / 8.7 / 9.5, 40 environments - / 10.1 / 10.8)
   const int cl_auto = s->n_env > 1 ? (s->fp64 ? (s->n_env <= 9 ? 16 : (s->n_env <= 48 ? 8 : 4)) : 4)
                                    : (V > 512 ? 8 : 1);
-  s->cluster = !block_mode ? 1 : (cl ? cl : cl_auto);
-  s->replan = block_mode && s->n_env > 1 && s->cluster > 1;
-  s->tiered = s->replan && (flags & VBD_TIERED) != 0;
-  // the wide tier: clusters twice the size of the split environments' (at
-  // most 16 blocks)
-  s->cluster_wide = s->tiered && (flags & VBD_TIERED_WIDE) && s->cluster < 16
-                        ? std::min(16, 2 * s->cluster)
-                        : 0;
+  auto set_cluster = [&](int automatic) {
+    s->cluster = !block_mode ? 1 : (cl ? cl : automatic);
+    s->replan = block_mode && s->n_env > 1 && s->cluster > 1;
+    s->tiered = s->replan && (flags & VBD_TIERED) != 0;
+    // the wide tier: clusters twice the size of the split environments' (at
+    // most 16 blocks)
+    s->cluster_wide = s->tiered && (flags & VBD_TIERED_WIDE) && s->cluster < 16
+                          ? std::min(16, 2 * s->cluster)
+                          : 0;
+  };
+  set_cluster(cl_auto);
   if (threads == 0)
     threads = block_mode ? (s->n_env > 1 && !s->fp64 ? 256 : 512)
                          : (mode == VBD_MODE_PERSIST ? 128 : 256);
@@ -1740,7 +1743,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
                            : (s->n_env > 1 ? 4 : domain_tpv(per));
     // one block per SM in persistent mode, whose warps are all the SM has: the
     // thread count is the domains' (a given one was meant for several blocks per SM)
-    if (!block_mode) s->threads = per <= 64 ? 256 : 512;
+    const int dom_threads = block_mode ? s->threads : (per <= 64 ? 256 : 512);
     DomLayout D;
     std::vector<int> first[3];
     for (int i = 0; i < 3 && D.fits; ++i)
@@ -1749,13 +1752,14 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
                           s->dom_smem[i]);
     int resident = 0;
     if (D.fits && !block_mode) {
-      if (bad(dom_occupancy(s->material, s->dom_tpv, s->threads, s->dom_smem[0][0], 1, true,
+      if (bad(dom_occupancy(s->material, s->dom_tpv, dom_threads, s->dom_smem[0][0], 1, true,
                             &resident),
               "persist occupancy"))
         err = 1;
     }
     if (!err && D.fits && (block_mode || resident * sms >= parts[0])) {
       s->by_domains = true;
+      s->threads = dom_threads;
       if (!block_mode) s->persist_blocks = s->ndom = parts[0];
       int posts = 0;
       bool split = false;
@@ -1789,6 +1793,10 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
         // blocks too large for two on an SM get the SM's warps
         if (2 * (s->smem_bytes + 7 * 1024) > 227 * 1024) s->threads = kDomMaxThreads;
       }
+    } else if (block_mode && s->n_env > 1) {
+      // the shape measured for env_step_kernel
+      set_cluster(4);
+      if (!threads_arg) s->threads = 256;
     }
   }
   if (!err && s->block_calls && !s->by_domains) {  // as without domains
@@ -2541,6 +2549,14 @@ int vbd_get_info(vbd_solver* s, vbd_info_t* info) {
   info->n_blocks = s->mode == VBD_MODE_PERSIST ? s->persist_blocks
                                                 : (int)(s->work.size() + s->work2.size() + s->work3.size());
   return VBD_OK;
+}
+
+const char* vbd_step_kernel(vbd_solver* s) {
+  if (!s) return "";
+  if (s->by_domains) return "domain_kernel";
+  return s->mode == VBD_MODE_BLOCK     ? "env_step_kernel"
+         : s->mode == VBD_MODE_PERSIST ? "persist_kernel"
+                                       : "color_kernel";
 }
 
 void* vbd_get_stream(vbd_solver* s) { return s ? (void*)s->stream : nullptr; }

@@ -311,10 +311,7 @@ class VBDSolver:
         return float(out[0])
 
     def info(self):
-        L = _lib.load()
-        inf = _lib.VBDInfo()
-        _lib.check(L.vbd_get_info(self._h, ctypes.byref(inf)))
-        return {n: getattr(inf, n) for n, _ in _lib.VBDInfo._fields_}
+        return _lib.info(self._h)
 
     @property
     def stream(self):
