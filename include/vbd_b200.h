@@ -128,9 +128,10 @@ int vbd_graph_coloring_gpu(const int32_t* tets, int n_tets, int32_t* coloring_ou
  *   coloring        int32   [max(tets)+1] colour per vertex, NULL = computed
  *   flags           VBD_MATERIAL_* | VBD_PRECISION_* | VBD_MODE_* | ...
  *   tpv             lanes per vertex (2, 4, 8, 16), 0 = pick automatically
+ *                   (fp64 in block and persistent mode runs at least 4)
  *   block_threads   threads per block, 0 = pick automatically.  In fp64 a launch whose
  *                   blocks each have an SM to themselves (persistent mode, large
- *                   environments) takes its own count, and batches at least 4 lanes
+ *                   environments) takes its own count
  *   device          CUDA device ordinal */
 int vbd_create(const double* rest_positions, int n_vertices, const int32_t* tets, int n_tets,
                const double* densities, const double* youngs_modulus,

@@ -207,3 +207,14 @@ def test_automatic_mode_keeps_a_cluster_size_asked_for():
     s = scenes.cantilever(40)
     sol = VBDSolver(**s.solver_kwargs(), damping_coefficient=0.0, cluster=4)
     assert sol.info()["mode"] == 0x100 and sol.info()["cluster"] == 4
+
+
+@pytest.mark.parametrize("opt", [dict(mode="persist"), dict(mode="block", cluster=1),
+                                 dict(mode="block", cluster=4)])
+def test_two_lanes_per_vertex_run_as_four(opt):
+    s = scenes.cantilever(21, 3, 2)
+    kw = dict(s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1000)
+    a, b = (VBDSolver(**kw, **opt, tpv=t, order_index=True) for t in (2, 4))
+    for _ in range(3):
+        x, y = (v.step(v.old_positions, 1e-3).numpy() for v in (a, b))
+        assert a.last_iterations == b.last_iterations and np.array_equal(x, y)

@@ -688,7 +688,6 @@ cudaError_t dom_dispatch(int material, bool split, F& f) {
 template <typename F>
 cudaError_t dom_dispatch(int material, int tpv, bool split, F& f) {
   switch (tpv) {
-    case 2: return dom_dispatch<2>(material, split, f);
     case 4: return dom_dispatch<4>(material, split, f);
     case 8: return dom_dispatch<8>(material, split, f);
     case 16: return dom_dispatch<16>(material, split, f);

@@ -1736,11 +1736,11 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     long long solved = 0;
     for (const EnvInfo& ei : s->L.env) solved += ei.nsolved;
     const int per = (int)(solved / s->n_env / std::max(1, s->n_env > 1 ? 1 : parts[0] + parts[1]));
-    // a batch's single blocks have registers for four lanes per vertex and more
-    // (with two, ten slots of a lane are held ahead: 83 instead of 79 us per
-    // sweep of 27K slots)
-    s->dom_tpv = tpv_given ? (s->n_env > 1 ? std::max(4, s->tpv) : s->tpv)
-                           : (s->n_env > 1 ? 4 : domain_tpv(per));
+    // Four lanes per vertex at least: with two, ten slots of a lane are held ahead and
+    // spill.  us per step with 2 / 4 lanes: 11^3 mass-spring on a cluster of 4 blocks 1065 /
+    // 838, on one block 1743 / 1712, 40x4x4 beam 676 / 467 and 832 / 701; 27K slots of a
+    // batch's environment 83 / 79 per sweep
+    s->dom_tpv = tpv_given ? std::max(4, s->tpv) : (s->n_env > 1 ? 4 : domain_tpv(per));
     // one block per SM in persistent mode, whose warps are all the SM has: the
     // thread count is the domains' (a given one was meant for several blocks per SM)
     const int dom_threads = block_mode ? s->threads : (per <= 64 ? 256 : 512);
