@@ -218,3 +218,25 @@ def test_two_lanes_per_vertex_run_as_four(opt):
     for _ in range(3):
         x, y = (v.step(v.old_positions, 1e-3).numpy() for v in (a, b))
         assert a.last_iterations == b.last_iterations and np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [2, 5, 37])
+@pytest.mark.parametrize("warm", [False, True])
+def test_plans_that_split_nothing_match_plain_blocks(n, warm):
+    """Small equal environments: the plan splits none, whatever the cluster size, and the step
+    is that of one block each, the padding of the last cluster included."""
+    import torch
+    from warpvbd_b200 import warmstart
+    envs = [scenes.mass_spring(2 + k % 2, 3) for k in range(n)]
+    a = BatchedVBDSolver(envs, dx_tol=1e-7, max_iter=1000)
+    b = BatchedVBDSolver(envs, dx_tol=1e-7, max_iter=1000, cluster=1)
+    assert a.info()["cluster"] > 1
+    if warm:
+        a.set_warmstart(warmstart.load())
+        b.set_warmstart(warmstart.load())
+    out = torch.empty((a.n_vertices, 3), dtype=torch.float64).pin_memory().numpy()
+    for _ in range(4):
+        assert np.array_equal(a.step(1e-3, out=out), b.step(1e-3))
+        assert a.info()["n_blocks"] - n < a.info()["cluster"]
+        assert a.info()["block_threads"] == b.info()["block_threads"]
+        assert np.array_equal(out, b.positions())

@@ -688,6 +688,11 @@ struct vbd_solver {
   bool tab_in_smem = false;   // kernels stage the record table in shared memory
   size_t persist_smem = 0;    // persistent mode: bytes of the staged table
   size_t smem_heavy = 0, smem_light = 0;
+  // by domains, not tiered: the current plan splits no environment, and runs as plain
+  // blocks of their own shared memory (largest single-block layout) and thread count
+  bool unsplit = false;
+  size_t smem_single = 0;
+  int split_threads = 512;  // threads of the non-tiered launch while it splits some
   std::vector<int4> work2;
   DevBuf<int4> d_work2;
   cudaStream_t aux = nullptr;
@@ -1078,6 +1083,8 @@ int upload_plan(vbd_solver* s, const int* iters) {
   s->work.swap(w);
   s->work2.swap(w2);
   s->work3.swap(w3);
+  s->unsplit = s->by_domains && !s->tiered && s->n_env > 1 &&
+               std::all_of(s->work.begin(), s->work.end(), [](const int4& x) { return x.z <= 1; });
   if (s->tiered) {
     s->smem_heavy = tier_smem(s, s->work);
     s->smem_light = tier_smem(s, s->work2);
@@ -1442,6 +1449,13 @@ cudaError_t block_occupancy(const vbd_solver* s, int threads, int cluster, int* 
                              out);
 }
 
+// Threads of the block mode's (non-tiered or light) launch under the current plan.
+int block_threads(const vbd_solver* s) {
+  return s->by_domains && s->mode == VBD_MODE_BLOCK && !s->tiered && s->cluster > 1 && !s->unsplit
+             ? s->split_threads
+             : s->threads;
+}
+
 // One block-mode launch over a work map.
 cudaError_t launch_block(const vbd_solver* s, const DevMesh& m, const StepParams& p,
                          const double* tol, const int4* work, int n_blocks, int cluster,
@@ -1790,8 +1804,11 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
         s->smem_bytes = 0;
         for (const auto& v : s->dom_smem)
           for (size_t x : v) s->smem_bytes = std::max(s->smem_bytes, x);
+        for (size_t x : s->dom_smem[0]) s->smem_single = std::max(s->smem_single, x);
         // blocks too large for two on an SM get the SM's warps
-        if (2 * (s->smem_bytes + 7 * 1024) > 227 * 1024) s->threads = kDomMaxThreads;
+        auto fills_sm = [](size_t x) { return 2 * (x + 7 * 1024) > 227 * 1024; };
+        s->split_threads = fills_sm(s->smem_bytes) ? kDomMaxThreads : s->threads;
+        if (fills_sm(s->n_env > 1 ? s->smem_single : s->smem_bytes)) s->threads = kDomMaxThreads;
       }
     } else if (block_mode && s->n_env > 1) {
       // the shape measured for env_step_kernel
@@ -1915,7 +1932,8 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
            bad(s->d_work3.alloc((size_t)s->n_env * s->cluster_wide), "work")))
         err = 1;
     } else {
-      if (bad(block_occupancy(s, s->threads, s->cluster, &occ), "occupancy"))
+      if (bad(block_occupancy(s, s->by_domains ? s->split_threads : s->threads, s->cluster, &occ),
+              "occupancy"))
         err = 1;
       s->capacity_blocks = s->cluster > 1 ? occ * s->cluster : occ * sms;
     }
@@ -2060,8 +2078,11 @@ int enqueue_step(vbd_solver* s, double dt, double tol, const double* tol_env, in
     NvtxRange nk("vbd_step_kernels");
     if (!s->tiered) {
       ++launches;
-      CUDA_TRY(launch_block(s, m, s->cur_params, dtol, s->d_work.p, (int)s->work.size(), s->cluster,
-                            s->threads, s->smem_bytes, st));
+      // an unsplit plan's blocks wait for none: no cluster, and the kernel without the
+      // handoff (8 environments of 40 vertices 497 -> 422 us, 100 of 600 419 -> 374)
+      CUDA_TRY(launch_block(s, m, s->cur_params, dtol, s->d_work.p, (int)s->work.size(),
+                            s->unsplit ? 1 : s->cluster, block_threads(s),
+                            s->unsplit ? s->smem_single : s->smem_bytes, st));
     } else {
       // the launches with the widest clusters first (they need whole groups
       // of free SMs): wide tier, split environments, then the single-block
@@ -2535,7 +2556,7 @@ int vbd_get_info(vbd_solver* s, vbd_info_t* info) {
   info->max_valence = s->L.max_valence;
   info->mode = s->mode;
   info->tpv = s->tpv;
-  info->block_threads = s->threads;
+  info->block_threads = block_threads(s);
   info->precision = s->prec;
   info->material = s->material;
   info->n_slots = s->L.n_slots;
