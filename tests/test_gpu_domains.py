@@ -240,3 +240,23 @@ def test_plans_that_split_nothing_match_plain_blocks(n, warm):
         assert a.info()["n_blocks"] - n < a.info()["cluster"]
         assert a.info()["block_threads"] == b.info()["block_threads"]
         assert np.array_equal(out, b.positions())
+
+
+@pytest.mark.parametrize("cube,n,threads", [
+    (2, 4, 128),     # a warp or two have chunks
+    (5, 4, 256),     # six
+    (7, 4, 512),     # sixteen
+    (7, 160, 256),   # more environments than SMs: two blocks on one
+    (2, 160, 128),
+    (15, 160, 512),  # an SM each: its shared memory is full
+])
+def test_default_thread_count_of_a_batch(cube, n, threads):
+    envs = [scenes.mass_spring(cube, 3)] * n
+    sol = BatchedVBDSolver(envs, dx_tol=1e-7, max_iter=1000, cluster=1)
+    assert sol.info()["block_threads"] == threads
+    its, x = _steps(sol, 2)
+    ref = BatchedVBDSolver(envs[:1], dx_tol=1e-7, max_iter=1000, cluster=1, tpv=4,
+                           block_threads=64)
+    for it in its:
+        assert (it == ref.step(1e-3)).all()
+    assert (x.reshape(n, -1, 3) == ref.positions()).all()

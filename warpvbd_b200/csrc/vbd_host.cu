@@ -1194,6 +1194,24 @@ struct DomLayout {
   }
 };
 
+// Threads of a batch's single-block environments: a warp for every chunk of the largest
+// colour, in powers of two from 128 to 512 threads (more warps only wait at the barrier
+// after each colour); at most 256 when there are more environments than SMs, so that two
+// blocks fit on one.  us per step with 128 / 256 / 512 threads: 100 environments of 135
+// vertices (4 chunks) 445 / 423 / 432, 100 of 225 (6) 425 / 339 / 349, 100 of 350 (9) 556 /
+// 428 / 374; 300 of 225 472 / 496 / 717, 300 of 350 651 / 589 / 734, 1,000 of 40 883 / 1683 /
+// 2935.
+int single_threads(const DomLayout& D, int n_env, int sms) {
+  int most = 1;
+  for (const DomInfo& di : D.dom)
+    if (di.nd == 1)
+      for (int c = di.cbase; c < di.cbase + di.ncolors; ++c)
+        most = std::max(most, D.color[c].chunk_end - D.color[c].chunk_begin);
+  int threads = 128;
+  while (threads < kDomMaxThreads && threads < 32 * most) threads *= 2;
+  return n_env > sms ? std::min(threads, 256) : threads;
+}
+
 void bisect(const std::vector<double>& x, const int* weight, std::vector<int>& ids, size_t begin,
             size_t end, int first, int parts, std::vector<int>& owner) {
   if (parts == 1) {
@@ -1808,6 +1826,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
         // blocks too large for two on an SM get the SM's warps
         auto fills_sm = [](size_t x) { return 2 * (x + 7 * 1024) > 227 * 1024; };
         s->split_threads = fills_sm(s->smem_bytes) ? kDomMaxThreads : s->threads;
+        if (!threads_arg && s->n_env > 1) s->threads = single_threads(D, s->n_env, sms);
         if (fills_sm(s->n_env > 1 ? s->smem_single : s->smem_bytes)) s->threads = kDomMaxThreads;
       }
     } else if (block_mode && s->n_env > 1) {
