@@ -30,6 +30,7 @@
 #include "vbd_domain.h"
 #include "vbd_persist.h"
 #include "vbd_noalloc.h"
+#include "vbd_plan.h"
 #include "vbd_setup.h"
 #include "vbd_warmstart.h"
 
@@ -666,6 +667,10 @@ struct vbd_solver {
   // once (a cluster needs its blocks in one GPC, so fewer than blocks / size)
   int max_clusters_split = 0, max_clusters_wide = 0;
   std::vector<double> env_work;  // incident slots per environment
+  // by domains: how much longer its slots take on one block, `cluster` and `cluster_wide`
+  // blocks (1, or kUnstagedSlots where a domain's records stay in global memory)
+  std::vector<double> slot_cost[3];
+  int sms = 0;
   // sweeps per environment for the plan.  Plain VBD's counts change slowly
   // from step to step: env_sweeps_decay = max(last, 0.95 x previous).  The
   // learned warm start's vary (consecutive-step correlation about 0.7 on the
@@ -917,6 +922,11 @@ size_t env_smem(const vbd_solver* s, const EnvInfo& ei, bool with_tab) {
 // then starts first.
 // I_C of the duration model: measured at C = 2, 4, 8, 16, linear in C between
 // those points (C = 3, 5-7, 9-15).
+constexpr double kDomA1 = 7200.0;
+// A slot visit with the records in global memory (5,000 distinct tets on one block: 77 us per
+// sweep, 58 by the constants above).
+constexpr double kUnstagedSlots = 1.45;
+
 double split_overhead(int C, bool fp64, bool by_domains) {
   static const double c[4] = {2.0, 4.0, 8.0, 16.0};
   static const double vm[4] = {10300.0, 11200.0, 12200.0, 16500.0};
@@ -945,7 +955,7 @@ void make_plan(const vbd_solver* s, const int* iters, std::vector<int4>& work,
   work2.clear();
   work3.clear();
   const bool f64 = s->prec == 2;
-  const double a1 = s->by_domains ? 7200.0 : (f64 ? 10200.0 : 8300.0);
+  const double a1 = s->by_domains ? kDomA1 : (f64 ? 10200.0 : 8300.0);
   const double aC = split_overhead(C, f64, s->by_domains);
   const double aW = Cw > 1 ? split_overhead(Cw, f64, s->by_domains) : 0.0;
   // high and mean estimates on one block, on C blocks and on Cw blocks
@@ -964,12 +974,15 @@ void make_plan(const vbd_solver* s, const int* iters, std::vector<int4>& work,
     k = std::max(1.0, k) + kw;
     km = std::max(1.0, km) + kw;
     const double slots = s->env_work[e];
-    d1[e] = k * (slots + a1);
-    dC[e] = C > 1 ? k * (slots / C + aC) : d1[e];
-    dW[e] = Cw > 1 ? k * (slots / Cw + aW) : dC[e];
-    m1[e] = km * (slots + a1);
-    mC[e] = C > 1 ? km * (slots / C + aC) : m1[e];
-    mW[e] = Cw > 1 ? km * (slots / Cw + aW) : mC[e];
+    auto cost = [&](int i) { return s->slot_cost[i].empty() ? 1.0 : s->slot_cost[i][e]; };
+    const double s1 = slots * cost(0) + a1, sC = slots / C * cost(1) + aC;
+    const double sW = Cw > 1 ? slots / Cw * cost(2) + aW : 0.0;
+    d1[e] = k * s1;
+    dC[e] = C > 1 ? k * sC : d1[e];
+    dW[e] = Cw > 1 ? k * sW : dC[e];
+    m1[e] = km * s1;
+    mC[e] = C > 1 ? km * sC : m1[e];
+    mW[e] = Cw > 1 ? km * sW : mC[e];
   }
   std::vector<int> order(n);
   for (int e = 0; e < n; ++e) order[e] = e;
@@ -1027,6 +1040,14 @@ void make_plan(const vbd_solver* s, const int* iters, std::vector<int4>& work,
     // a wider cluster for the next environment cannot beat this once the
     // wide jobs alone are the longest
     if (h1 < n && t_wide >= best_t) break;
+  }
+  if (s->by_domains && !s->tiered) {  // one launch: the order in which it starts counts
+    std::vector<double> one(n), split(n);
+    for (int i = 0; i < n; ++i) {
+      one[i] = d1[order[i]];
+      split[i] = dC[order[i]];
+    }
+    best_h = split_count(one, split, C, s->capacity_blocks / C, s->sms, best_h);
   }
   std::stable_sort(order.begin(), order.begin() + best_h1,
                    [&](int a, int b) { return dW[a] > dW[b]; });
@@ -1818,6 +1839,14 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
               "domains"))
         err = 1;
       cudaStreamSynchronize(st);  // D and first go out of scope
+      s->sms = sms;
+      for (int i = 0; i < 3; ++i)
+        for (size_t e = 0; e < first[i].size(); ++e) {
+          bool staged = true;
+          for (int d = first[i][e]; d < first[i][e] + D.dom[first[i][e]].nd; ++d)
+            staged = staged && (D.dom[d].flags & kDomRecords);
+          s->slot_cost[i].push_back(staged ? 1.0 : kUnstagedSlots);
+        }
       if (block_mode) {
         s->smem_bytes = 0;
         for (const auto& v : s->dom_smem)
