@@ -260,3 +260,22 @@ def test_default_thread_count_of_a_batch(cube, n, threads):
     for it in its:
         assert (it == ref.step(1e-3)).all()
     assert (x.reshape(n, -1, 3) == ref.positions()).all()
+
+
+def test_default_cluster_size_of_a_batch():
+    """Seven clusters of 16 blocks fit a B200: six environments take them, eight equal ones
+    with many distinct tets take eight blocks each and start together."""
+    rng = np.random.default_rng(0)
+    heavy = []
+    for _ in range(8):
+        s = scenes.mass_spring(10, 6)
+        s.vertices = s.vertices + rng.uniform(-0.08, 0.08, s.vertices.shape) * s.meta["voxel"]
+        heavy.append(s)
+    for envs, cluster in ((scenes.env_batch(6, seed=0), 16), (heavy, 8)):
+        a = BatchedVBDSolver(envs, dx_tol=1e-7, max_iter=1000)
+        b = BatchedVBDSolver(envs, dx_tol=1e-7, max_iter=1000, cluster=1)
+        assert a.info()["cluster"] == cluster
+        for _ in range(3):
+            assert np.array_equal(a.step(1e-3), b.step(1e-3))
+        assert a.info()["n_blocks"] > len(envs)
+        assert np.array_equal(a.positions(), b.positions())

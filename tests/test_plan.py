@@ -24,6 +24,10 @@ double launch_time(const double* a, const double* b, int n, int h, int C, int k,
 int split_count(const double* a, const double* b, int n, int C, int k, int sms, int bound) {
   return vbd::split_count(v(a, n), v(b, n), C, k, sms, bound);
 }
+int pick_cluster(int preferred, const int* clusters, const double* time) {
+  return vbd::pick_cluster(preferred, [&](int C) { return clusters[C]; },
+                           [&](int C, int) { return time[C]; });
+}
 }
 """)
     subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{CSRC}",
@@ -89,3 +93,21 @@ def test_the_choice_is_never_worse_than_its_candidates(lib, seed):
     bound, clusters = int(rng.integers(0, n + 1)), int(rng.integers(1, 74))
     h, t = _split(lib, one, split, C, clusters, bound)
     assert t[h] <= min(t[0], t[n], t[bound]) * 1.002
+
+
+@pytest.mark.parametrize("preferred,clusters,time,want", [
+    (16, {16: 7, 8: 16, 4: 33, 2: 70}, {16: 10, 8: 10, 4: 10, 2: 10}, 16),
+    (16, {16: 7, 8: 16, 4: 33, 2: 70}, {16: 25, 8: 13, 4: 15, 2: 24}, 8),
+    (8, {8: 16, 4: 33, 2: 70}, {8: 10, 4: 9.5, 2: 9.2}, 8),   # within the model's error
+    (16, {16: 0, 8: 16, 4: 33, 2: 70}, {16: 1, 8: 10, 4: 10, 2: 10}, 8),  # none resident
+    (16, {16: 0, 8: 0, 4: 0, 2: 3}, {16: 1, 8: 1, 4: 1, 2: 9}, 2),
+    (4, {4: 0, 2: 0}, {4: 1, 2: 1}, 1),
+])
+def test_default_cluster_size(lib, preferred, clusters, time, want):
+    k, t = np.zeros(17, np.int32), np.zeros(17)
+    for C in clusters:
+        k[C], t[C] = clusters[C], time[C]
+    lib.pick_cluster.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_int32),
+                                 ctypes.POINTER(ctypes.c_double)]
+    assert lib.pick_cluster(preferred, k.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)),
+                            _p(t)) == want

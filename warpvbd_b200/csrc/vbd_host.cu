@@ -939,6 +939,33 @@ double split_overhead(int C, bool fp64, bool by_domains) {
   return v[3];
 }
 
+// Predicted time (slot visits) of one sweep of every environment in one launch by domains
+// that may split some over clusters of C, `clusters` of which can be resident.  Whether a
+// part's records are staged is guessed: 1.4 times its share of the tets, and 1.6 times its
+// share of the vertices, are its own and its halo's.
+double predicted_time(const Layout& L, int C, int clusters, int sms) {
+  std::vector<std::pair<double, double>> t;
+  for (const EnvInfo& e : L.env) {
+    auto slots = [&](int parts) {
+      const double own = 1.0 / parts, grow = parts > 1 ? 1.0 : 0.0;
+      const int nrec = std::min<int>(e.nrec, (int)((1.0 + 0.4 * grow) * own * e.ntets));
+      const int nloc = (int)((1.0 + 0.6 * grow) * own * e.nv);
+      const bool staged = dom_smem(nloc, nrec, 0, 0, kDomRecords) <= kDomMaxSmem;
+      return 4.0 * e.ntets * own * (staged ? 1.0 : kUnstagedSlots);
+    };
+    t.emplace_back(slots(1) + kDomA1, slots(C) + split_overhead(C, true, true));
+  }
+  std::sort(t.begin(), t.end(), std::greater<std::pair<double, double>>());
+  std::vector<double> one, split;
+  for (const auto& x : t) {
+    one.push_back(x.first);
+    split.push_back(x.second);
+  }
+  double time = 0.0;
+  split_count(one, split, C, clusters, sms, 0, &time);
+  return time;
+}
+
 // With the wide tier (VBD_TIERED_WIDE, tiered mode) the longest split
 // environments may instead take a cluster of Cw = cluster_wide blocks, in a
 // third launch: the planner tries every split of the environments, longest
@@ -1617,7 +1644,9 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   }
   // fp64: as many blocks per environment as there are SMs to go round (kernel ms
   // of three steps with clusters of 16 / 8 / 4: 6 uneven environments 5.0 / 6.1 /
-  // 9.0, 16 environments 8.5 / 8.7 / 9.5, 40 environments - / 10.1 / 10.8)
+  // 9.0, 16 environments 8.5 / 8.7 / 9.5, 40 environments - / 10.1 / 10.8), or smaller ones
+  // (pick_cluster: only seven clusters of 16 fit; us per step with 16 / 8: 8 equal irregular
+  // environments of 1,355 vertices 860 / 550)
   const int cl_auto = s->n_env > 1 ? (s->fp64 ? (s->n_env <= 9 ? 16 : (s->n_env <= 48 ? 8 : 4)) : 4)
                                    : (V > 512 ? 8 : 1);
   auto set_cluster = [&](int automatic) {
@@ -1776,6 +1805,31 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const bool sort_records = (flags & VBD_ORDER_INDEX) == 0;
+    if (block_mode && s->n_env > 1 && !cl) {
+      // uneven environments keep the size above: their largest also take the most sweeps,
+      // which are not known yet (9 / 40 / 100 uneven environments on smaller clusters 1717 ->
+      // 1851, 2358 -> 2815, 1413 -> 1656 us per step)
+      double most = 0.0, all = 0.0;
+      for (const EnvInfo& e : s->L.env) {
+        most = std::max(most, (double)e.ntets);
+        all += e.ntets;
+      }
+      const bool even = most * s->n_env <= 1.5 * all;
+      set_cluster(pick_cluster(
+          s->cluster,
+          [&](int C) {
+            int k = 0;
+            if (dom_occupancy(s->material, std::max(4, s->tpv), kDomMaxThreads, kDomMaxSmem, C,
+                              true, &k) != cudaSuccess) {
+              cudaGetLastError();
+              return 0;
+            }
+            return k;
+          },
+          [&](int C, int k) {
+            return even && !(flags & VBD_TIERED) ? predicted_time(s->L, C, k, sms) : 0.0;
+          }));
+    }
     // layouts: persistent mode one; block mode 1, cluster and cluster_wide domains
     // (a single environment in a cluster is never on one block)
     int parts[3] = {0, 0, 0};

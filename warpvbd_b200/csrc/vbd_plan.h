@@ -66,4 +66,24 @@ inline int split_count(const std::vector<double>& d1, const std::vector<double>&
   return best;
 }
 
+// Blocks per cluster of a batch whose caller names none: `preferred`, or half of it and so
+// on down to 2 where no cluster of the larger size can be resident, or where the smaller is
+// predicted to be faster by more than the model's error (a tenth).  clusters(C): how many can
+// be resident; time(C, clusters): the predicted launch time.  1 if no cluster can be.
+template <class Clusters, class Time>
+int pick_cluster(int preferred, Clusters clusters, Time time) {
+  int best = 1;
+  double best_t = 1e300;
+  for (int C = preferred; C >= 2; C /= 2) {
+    const int k = clusters(C);
+    if (k < 1) continue;
+    const double t = time(C, k);
+    if (best == 1 || t < 0.9 * best_t) {
+      best = C;
+      best_t = t;
+    }
+  }
+  return best;
+}
+
 }  // namespace vbd
