@@ -225,7 +225,7 @@ int vbd_get_color_groups(vbd_solver* s, int32_t* table, int* n_colors, int* max_
 /* Sizes and the configuration the solver runs with. */
 typedef struct vbd_info_t {
   int n_vertices, n_tets, n_env, n_colors, max_valence;
-  int mode, tpv, block_threads, precision, material;
+  int mode, tpv, block_threads, precision, material; /* tpv, block_threads: as launched */
   long long n_slots, n_slot_records; /* incident (vertex, tet) pairs; padded records */
   long long device_bytes;
   int n_unique_records; /* entries of the shared slot-record table */

@@ -57,6 +57,30 @@ def test_cache_roundtrip_and_key_sensitivity(tmp_path):
     assert autotune.lookup(k1, path) == cfg
 
 
+def test_shapes_that_launch_alike_are_timed_once():
+    """block_threads that a launch replaces, two lanes that run as four: one measurement each,
+    and the result names the launch."""
+    spaces = {"persist": {"tpv": [2, 4, 8], "block_threads": [256, 512], "order_index": [False]}}
+    shapes, timed = autotune._Shapes(), []
+
+    def evaluate(cfg):
+        info = {"mode": 0x400, "kernel": "domain_kernel", "tpv": max(4, cfg["tpv"]),
+                "block_threads": 512, "cluster": 1}
+
+        def measure():
+            timed.append(info["tpv"])
+            return {4: 1.0, 8: 2.0}[info["tpv"]] - 0.01 * len(timed)  # noise: later is faster
+        return shapes.cost(cfg, info, measure)
+    best, cost, log = autotune.search_families(spaces, evaluate)
+    assert timed == [4, 8] and len(log) > len(timed)
+    assert autotune._kwargs(shapes.launched(best)) == {
+        "mode": "persist", "tpv": 4, "block_threads": 512, "cluster": 0, "order_index": False}
+
+
+def test_default_spaces_reach_the_automatic_shape():
+    assert 0 in autotune.SINGLE_SPACE["persist"]["tpv"]
+
+
 def test_committed_table_is_valid_json():
     import json
     import os

@@ -1,0 +1,43 @@
+"""info() describes what is launched and allocated."""
+import numpy as np
+import pytest
+
+from warpvbd_b200 import BatchedVBDSolver, VBDSolver, autotune, scenes
+
+pytestmark = pytest.mark.gpu
+KW = dict(dx_tol=1e-7, max_iter=1000)
+
+
+def test_lanes_and_threads_as_launched():
+    envs = [scenes.mass_spring(4, 3)] * 3
+    assert BatchedVBDSolver(envs, **KW, tpv=2).info()["tpv"] == 4
+    assert BatchedVBDSolver(envs, **KW, tpv=2, precision="mixed").info()["tpv"] == 2
+    s = scenes.cantilever(20)
+    sol = VBDSolver(**s.solver_kwargs(), **KW, damping_coefficient=0.0, mode="persist",
+                    block_threads=64)
+    assert sol.info()["tpv"] == 32 and sol.info()["block_threads"] == 256
+
+
+def test_device_bytes_count_the_domains():
+    """Slots, records and positions of the domains lie beside the solver's: three layouts in a
+    batch with a wide tier.  48 bytes a vertex go to the handoff, 8 to every slot."""
+    envs = [scenes.mass_spring(6, 5)] * 4
+    one = BatchedVBDSolver(envs, **KW, cluster=1).info()
+    wide = BatchedVBDSolver(envs, **KW, cluster=4, tiered=True).info()
+    graph = VBDSolver(**envs[0].solver_kwargs(), **KW, damping_coefficient=0.0,
+                      mode="graph").info()
+    n_slots = wide["n_slots"]
+    assert one["device_bytes"] > 4 * graph["device_bytes"] + 8 * n_slots
+    assert wide["device_bytes"] - one["device_bytes"] > 2 * 8 * n_slots + 48 * wide["n_vertices"]
+
+
+def test_tuned_shape_is_no_slower_than_the_automatic_one(tmp_path):
+    """The tuner's space holds the automatic shape, on a mesh small enough that it once left
+    the persistent mode out: what it returns is that shape or one that beat it."""
+    kw = scenes.cantilever(20).solver_kwargs()
+    auto = VBDSolver(**kw, **KW, damping_coefficient=0.0).info()
+    cfg = autotune.tune_single(kw, refresh=True, cache_path=str(tmp_path / "t.json"))
+    ran = VBDSolver(**kw, **KW, damping_coefficient=0.0, **cfg).info()
+    assert auto["mode"] == 0x400
+    assert cfg["mode"] in ("persist", "block") and cfg["block_threads"] == ran["block_threads"]
+    assert np.isfinite([ran["tpv"]]).all() and (cfg["tpv"] in (0, ran["tpv"]))

@@ -50,7 +50,8 @@ PACKAGE_TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data",
 SINGLE_SPACE = {
     "block": {"tpv": [2, 4, 8, 16], "block_threads": [256, 512, 128],
               "cluster": [1, 2, 4, 8, 16], "order_index": [False, True]},
-    "persist": {"tpv": [4, 2, 8, 16], "block_threads": [256, 512, 128],
+    # 0: the automatic choice, which in fp64 takes 32 lanes on small domains
+    "persist": {"tpv": [0, 4, 2, 8, 16], "block_threads": [256, 512, 128],
                 "order_index": [False, True]},
     "graph": {"tpv": [4, 2, 8, 16], "order_index": [False, True]},
 }
@@ -59,10 +60,6 @@ BATCH_SPACE = {
               "cluster": [4, 8, 2, 16], "tpv": [4, 2, 8],
               "block_threads": [256, 128, 512], "order_index": [False, True]},
 }
-# Meshes of at most this many vertices are tuned among the block shapes only: the
-# persistent mode is some 30 % faster there, but holds a dozen SMs for a step that
-# is as short as the host's time per step.
-PERSIST_MIN_VERTICES = 256
 # Shared memory a block-mode step may use (bytes), and per vertex.
 BLOCK_SMEM_LIMIT = 227 * 1024 - 2048
 STATE_BYTES = {"fp32": 12, "mixed": 24, "fp64": 24}
@@ -200,6 +197,27 @@ def _time_solver(sol, step, steps, warmup, batched):
     return ms / steps if batched else ms / max(1, sweeps)
 
 
+class _Shapes:
+    """Costs by the shape a solver launches (its info()), which may differ from the one asked
+    for: candidates that launch alike are timed once, so that noise does not choose among
+    them, and the result names what ran."""
+
+    def __init__(self):
+        self.costs, self.ran = {}, {}
+
+    def cost(self, cfg, info, measure):
+        ran = {k: info[k] for k in ("tpv", "block_threads") if cfg.get(k)}
+        self.ran[tuple(sorted(cfg.items()))] = ran
+        key = (info["mode"], info["kernel"], info["tpv"], info["block_threads"], info["cluster"],
+               *(cfg.get(k) for k in ("order_index", "tiered", "wide_tier")))
+        if key not in self.costs:
+            self.costs[key] = measure()
+        return self.costs[key]
+
+    def launched(self, cfg):
+        return dict(cfg, **self.ran.get(tuple(sorted(cfg.items())), {}))
+
+
 def _fits_block(n_vertices, precision):
     return n_vertices * STATE_BYTES[precision] <= BLOCK_SMEM_LIMIT
 
@@ -224,8 +242,8 @@ def tune_single(solver_kwargs, *, material="snh", precision="fp64", device="cuda
             return hit
     if spaces is None:
         spaces = {m: s for m, s in SINGLE_SPACE.items()
-                  if (m != "block" or _fits_block(X.shape[0], precision))
-                  and (m != "persist" or X.shape[0] > PERSIST_MIN_VERTICES)}
+                  if m != "block" or _fits_block(X.shape[0], precision)}
+    shapes = _Shapes()
 
     def evaluate(cfg):
         mode = cfg["mode"]
@@ -240,8 +258,9 @@ def tune_single(solver_kwargs, *, material="snh", precision="fp64", device="cuda
                 print("skip", cfg, str(e)[:80])
             return math.inf
         try:
-            c = _time_solver(sol, lambda: sol.step(sol.old_positions, dt, blocking=False),
-                             steps, warmup, False)
+            c = shapes.cost(cfg, sol.info(), lambda: _time_solver(
+                sol, lambda: sol.step(sol.old_positions, dt, blocking=False), steps, warmup,
+                False))
         finally:
             sol.close()
         if verbose:
@@ -250,7 +269,7 @@ def tune_single(solver_kwargs, *, material="snh", precision="fp64", device="cuda
 
     t0 = time.perf_counter()
     best, cost, log = search_families(spaces, evaluate)
-    cfg = _kwargs(best)
+    cfg = _kwargs(shapes.launched(best))
     store(key, cfg, {"ms_per_sweep": cost, "device": name, "evaluated": len(log),
                      "tune_s": round(time.perf_counter() - t0, 1),
                      "n_vertices": int(X.shape[0]), "n_tets": int(T.shape[0])}, cache_path)
@@ -289,6 +308,7 @@ def tune_batched(envs, *, material="snh", precision="fp64", device="cuda", dt=1e
         if hit is not None:
             return hit
     spaces = spaces or BATCH_SPACE
+    shapes = _Shapes()
 
     def evaluate(cfg):
         args = {k: cfg[k] for k in ("tpv", "block_threads", "cluster", "order_index", "tiered",
@@ -303,7 +323,8 @@ def tune_batched(envs, *, material="snh", precision="fp64", device="cuda", dt=1e
                 print("skip", cfg, str(e)[:80])
             return math.inf
         try:
-            c = _time_solver(sol, lambda: sol.step(dt, blocking=False), steps, warmup, True)
+            c = shapes.cost(cfg, sol.info(), lambda: _time_solver(
+                sol, lambda: sol.step(dt, blocking=False), steps, warmup, True))
         finally:
             sol.close()
         if verbose:
@@ -312,7 +333,7 @@ def tune_batched(envs, *, material="snh", precision="fp64", device="cuda", dt=1e
 
     t0 = time.perf_counter()
     best, cost, log = search_families(spaces, evaluate)
-    cfg = {k: v for k, v in _kwargs(best).items() if k != "mode"}
+    cfg = {k: v for k, v in _kwargs(shapes.launched(best)).items() if k != "mode"}
     cfg["tiered"] = bool(best.get("tiered", False))
     cfg["wide_tier"] = cfg["tiered"] and bool(best.get("wide_tier", True))
     store(key, cfg, {"ms_per_step": cost, "device": name, "evaluated": len(log),

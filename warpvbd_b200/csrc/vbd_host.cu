@@ -2057,6 +2057,10 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   s->device_bytes += (long long)(4 * sb + s->d_X.n * 8 + s->d_io.n * 8);
   s->device_bytes += (long long)(s->d_valence.n * 4 + s->d_map.n * 4);
   s->device_bytes += (long long)(s->d_tet_slot.n * sizeof(int4) + s->d_tet_owner.n * 4);
+  auto bytes = [](const auto&... b) { return (long long)((b.n * sizeof(*b.p)) + ...); };
+  s->device_bytes += bytes(s->d_dom, s->d_dom_color, s->d_dom_chunk, s->d_dom_slot, s->d_dom_local,
+                           s->d_dom_rec, s->d_dom_tet, s->d_dom_tet_owner, s->d_dom_mail,
+                           s->d_dom_post, s->d_dom_first[0], s->d_dom_first[1], s->d_dom_first[2]);
   *out = s;
   return VBD_OK;
 }
@@ -2657,7 +2661,7 @@ int vbd_get_info(vbd_solver* s, vbd_info_t* info) {
   info->n_colors = s->L.max_colors;
   info->max_valence = s->L.max_valence;
   info->mode = s->mode;
-  info->tpv = s->tpv;
+  info->tpv = s->by_domains ? s->dom_tpv : s->tpv;
   info->block_threads = block_threads(s);
   info->precision = s->prec;
   info->material = s->material;
