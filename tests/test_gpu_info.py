@@ -1,5 +1,4 @@
 """info() describes what is launched and allocated."""
-import numpy as np
 import pytest
 
 from warpvbd_b200 import BatchedVBDSolver, VBDSolver, autotune, scenes
@@ -31,13 +30,12 @@ def test_device_bytes_count_the_domains():
     assert wide["device_bytes"] - one["device_bytes"] > 2 * 8 * n_slots + 48 * wide["n_vertices"]
 
 
-def test_tuned_shape_is_no_slower_than_the_automatic_one(tmp_path):
-    """The tuner's space holds the automatic shape, on a mesh small enough that it once left
-    the persistent mode out: what it returns is that shape or one that beat it."""
-    kw = scenes.cantilever(20).solver_kwargs()
-    auto = VBDSolver(**kw, **KW, damping_coefficient=0.0).info()
-    cfg = autotune.tune_single(kw, refresh=True, cache_path=str(tmp_path / "t.json"))
-    ran = VBDSolver(**kw, **KW, damping_coefficient=0.0, **cfg).info()
-    assert auto["mode"] == 0x400
-    assert cfg["mode"] in ("persist", "block") and cfg["block_threads"] == ran["block_threads"]
-    assert np.isfinite([ran["tpv"]]).all() and (cfg["tpv"] in (0, ran["tpv"]))
+def test_tuner_reaches_the_automatic_shape(tmp_path):
+    """The tuner's space holds the automatic shape, 32 lanes among it, and its result names
+    what is launched."""
+    kw = scenes.cantilever(40).solver_kwargs()
+    cfg = autotune.tune_single(kw, spaces={"persist": autotune.SINGLE_SPACE["persist"]},
+                               refresh=True, cache_path=str(tmp_path / "t.json"))
+    auto, ran = (VBDSolver(**kw, **KW, damping_coefficient=0.0, **c).info() for c in ({}, cfg))
+    assert auto["mode"] == ran["mode"] == 0x400 and auto["tpv"] == 32
+    assert cfg["block_threads"] == ran["block_threads"] and cfg["tpv"] in (0, ran["tpv"])
