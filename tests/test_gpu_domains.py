@@ -279,3 +279,17 @@ def test_default_cluster_size_of_a_batch():
             assert np.array_equal(a.step(1e-3), b.step(1e-3))
         assert a.info()["n_blocks"] > len(envs)
         assert np.array_equal(a.positions(), b.positions())
+
+
+@pytest.mark.parametrize("shape", [(63, 1, 1), (64, 1, 1), (65, 1, 1), (127, 1, 1), (128, 1, 1),
+                                   (129, 1, 1), (40, 4, 4)])
+def test_domains_set_up_in_groups_are_those_of_one(shape):
+    """Host threads take groups of domains from 256 solved vertices on (252, 256, 260; 508,
+    512, 516; 1,000): the step is that of one domain, bit for bit at equal lanes."""
+    s = scenes.cantilever(*shape)
+    kw = dict(s.solver_kwargs(), damping_coefficient=0.0, dx_tol=1e-7, max_iter=1000, tpv=4)
+    a, b = VBDSolver(**kw, mode="persist"), VBDSolver(**kw, mode="block", cluster=1)
+    assert a.info()["n_blocks"] > 1
+    for _ in range(3):
+        x, y = (v.step(v.old_positions, 1e-3).numpy() for v in (a, b))
+        assert a.last_iterations == b.last_iterations and np.array_equal(x, y)

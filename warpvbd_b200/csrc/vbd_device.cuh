@@ -213,14 +213,19 @@ __device__ __forceinline__ double4 ldg_row(const double4* p) {
 // a record is 96 bytes, so without it the same half of eight consecutive
 // records would fall into four of the eight 16-byte bank groups (70 instead of
 // 50 shared-memory wavefronts per 32 slots on the 11^3 mass-spring).
-__device__ __forceinline__ void stage_table(unsigned char* dst, const RecTab<double>& t, int nrec) {
+// at(record, row): where the row lies in global memory.
+template <class At>
+__device__ __forceinline__ void stage_rows(unsigned char* dst, int nrec, At at) {
   for (int i = threadIdx.x; i < 3 * nrec; i += blockDim.x) {
-    const double4 v = ldg_row(t.g + i);
+    const double4 v = ldg_row(at(i / 3, i % 3));
     double2* d = reinterpret_cast<double2*>(dst) + 2 * i;
     const int sw = (i / 3 >> 2) & 1;
     d[sw] = make_double2(v.x, v.y);
     d[sw ^ 1] = make_double2(v.z, v.w);
   }
+}
+__device__ __forceinline__ void stage_table(unsigned char* dst, const RecTab<double>& t, int nrec) {
+  stage_rows(dst, nrec, [&](int rec, int row) { return t.g + 3 * (size_t)rec + row; });
 }
 __device__ __forceinline__ void stage_table(unsigned char* dst, const RecTab<float>& t, int nrec) {
   float4* d = reinterpret_cast<float4*>(dst);

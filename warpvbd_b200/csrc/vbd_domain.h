@@ -16,7 +16,7 @@ struct DomInfo {
   int nd, rank;      // domains of the environment, and this one's number
   int lbase;         // first entry of the domain in DomDev::local
   int nown, nloc;    // own vertices; all local vertices
-  int rbase, nrec;   // its records in DomDev::rec (three double4 each)
+  int rbase, nrec;   // its records: from DomDev::rec_id (kDomRecords) or in DomDev::rec
   int tbase, ntets;  // its tets in DomDev::tet_slot (those whose owner is its own)
   int qbase, nchunk;   // its chunks
   int cbase, ncolors;  // its colours
@@ -58,7 +58,8 @@ struct DomDev {
   const ushort4* slot;       // (n0, n1, n2, 4 x record + place), local ids
   const int2* local;         // (renumbered vertex id, or its complement when other domains
                              // read the vertex; incident tets)
-  const double4* rec;
+  const int* rec_id;         // staged records: places in the environment's table
+  const double4* rec;        // records read from global memory, three double4 each
   const int4* tet_slot;      // owner slot of every tet, local ids
   const int* tet_owner;      // its owner's local id
   ulonglong2* mail;          // [vertices][3]: (coordinate bits, tag)

@@ -647,16 +647,9 @@ struct vbd_solver {
   int ndom = 0, dom_tpv = 0;
   unsigned dom_seq = 0;
   std::vector<size_t> dom_smem[3];  // per environment
-  DevBuf<int> d_dom_first[3];
-  DevBuf<DomInfo> d_dom;
-  DevBuf<DomColor> d_dom_color;
-  DevBuf<DomChunk> d_dom_chunk;
-  DevBuf<ushort4> d_dom_slot;
-  DevBuf<int2> d_dom_local;
-  DevBuf<double> d_dom_rec;
-  DevBuf<int4> d_dom_tet;
-  DevBuf<int> d_dom_tet_owner;
-  DevBuf<ulonglong2> d_dom_mail, d_dom_post;
+  DevBuf<unsigned char> d_dom;  // all of their arrays
+  DomDev dom{};                 // pointers into it
+  const int* dom_first[3] = {nullptr, nullptr, nullptr};  // first domain of every environment
   unsigned dom_abort_seen = 0;  // the abort word when the last step was finished
   PersistLimits wait_limits{1ll << 26, 2000000000ull};  // every grid-barrier wait
   // block-mode work map: (environment, rank, group size) per thread block
@@ -842,17 +835,7 @@ void free_solver(vbd_solver* s) {
   s->d_nbr_off.release();
   s->d_nbr_idx.release();
   s->d_epoch.release();
-  for (auto& f : s->d_dom_first) f.release();
   s->d_dom.release();
-  s->d_dom_color.release();
-  s->d_dom_chunk.release();
-  s->d_dom_slot.release();
-  s->d_dom_local.release();
-  s->d_dom_rec.release();
-  s->d_dom_tet.release();
-  s->d_dom_tet_owner.release();
-  s->d_dom_mail.release();
-  s->d_dom_post.release();
   if (s->h_iters) cudaFreeHost(s->h_iters);
   if (s->h_status) cudaFreeHost(s->h_status);
   if (s->h_dxmax) cudaFreeHost(s->h_dxmax);
@@ -1212,21 +1195,27 @@ struct DomLayout {
   std::vector<DomChunk> chunk;
   std::vector<ushort4> slot;
   std::vector<int2> local;
+  std::vector<int> rec_id;
   std::vector<double> rec;
   std::vector<int4> tet_slot;
   std::vector<int> tet_owner;
   bool fits = true;  // positions in a block's shared memory, ids in 16 bits
 
   // Appends another layout, its offsets moved behind this one's.
-  void append(const DomLayout& o) {
+  void append(DomLayout& o) {
+    if (dom.empty()) {
+      std::swap(*this, o);
+      fits = fits && o.fits;
+      return;
+    }
     const int nd = (int)dom.size(), nc = (int)color.size(), nq = (int)chunk.size();
     const int nb = (int)(slot.size() / 32), nl = (int)local.size(), nr = (int)(rec.size() / 12);
-    const int nt = (int)tet_slot.size();
+    const int nt = (int)tet_slot.size(), ni = (int)rec_id.size();
     fits = fits && o.fits;
     dom.insert(dom.end(), o.dom.begin(), o.dom.end());
     for (size_t i = nd; i < dom.size(); ++i) {
       dom[i].lbase += nl;
-      dom[i].rbase += nr;
+      dom[i].rbase += (dom[i].flags & kDomRecords) ? ni : nr;
       dom[i].tbase += nt;
       dom[i].qbase += nq;
       dom[i].cbase += nc;
@@ -1236,6 +1225,7 @@ struct DomLayout {
     color.insert(color.end(), o.color.begin(), o.color.end());
     slot.insert(slot.end(), o.slot.begin(), o.slot.end());
     local.insert(local.end(), o.local.begin(), o.local.end());
+    rec_id.insert(rec_id.end(), o.rec_id.begin(), o.rec_id.end());
     rec.insert(rec.end(), o.rec.begin(), o.rec.end());
     tet_slot.insert(tet_slot.end(), o.tet_slot.begin(), o.tet_slot.end());
     tet_owner.insert(tet_owner.end(), o.tet_owner.begin(), o.tet_owner.end());
@@ -1260,46 +1250,82 @@ int single_threads(const DomLayout& D, int n_env, int sms) {
   return n_env > sms ? std::min(threads, 256) : threads;
 }
 
-void bisect(const std::vector<double>& x, const int* weight, std::vector<int>& ids, size_t begin,
-            size_t end, int first, int parts, std::vector<int>& owner) {
-  if (parts == 1) {
-    for (size_t i = begin; i < end; ++i) owner[ids[i]] = first;
-    return;
+// Recursive bisection of vertices into parts of about equal weight, across the longest side
+// of what is left.  The vertices are sorted by each coordinate once (and by id where equal);
+// every cut keeps the three orders, so that no level sorts again (1,808 vertices in 148 parts
+// 1.4 -> 0.3 ms).
+struct Bisection {
+  const std::vector<double>& x;  // positions, three a vertex
+  const int* weight;
+  std::vector<int>& owner;  // of every vertex: its part
+  std::vector<int> order[3], spare;
+  std::vector<char> left_side;
+
+  Bisection(const std::vector<double>& x, const int* weight, int n, std::vector<int>& owner)
+      : x(x), weight(weight), owner(owner), spare(n), left_side(n) {
+    for (int c = 0; c < 3; ++c) sort_by(c, n);
   }
-  double lo[3], hi[3];
-  for (int c = 0; c < 3; ++c) {
-    lo[c] = 1e300;
-    hi[c] = -1e300;
-  }
-  long long total = 0;
-  for (size_t i = begin; i < end; ++i) {
-    for (int c = 0; c < 3; ++c) {
-      lo[c] = std::min(lo[c], x[3 * (size_t)ids[i] + c]);
-      hi[c] = std::max(hi[c], x[3 * (size_t)ids[i] + c]);
+
+  // Radix sort of the ids by coordinate c: eight stable passes over a byte of the key each,
+  // those left out in which all keys agree.
+  void sort_by(int c, int n) {
+    std::vector<uint64_t> key(n);
+    for (int v = 0; v < n; ++v) {
+      const double d = x[3 * (size_t)v + c] + 0.0;  // -0 and 0 are equal
+      uint64_t u;
+      std::memcpy(&u, &d, sizeof u);
+      key[v] = u >> 63 ? ~u : u | 1ull << 63;  // unsigned order = the doubles'
     }
-    total += weight[ids[i]];
+    std::vector<int>& ids = order[c];
+    ids.resize(n);
+    for (int i = 0; i < n; ++i) ids[i] = i;
+    for (int shift = 0; shift < 64; shift += 8) {
+      size_t at[257] = {};
+      for (uint64_t k : key) ++at[(k >> shift & 255) + 1];
+      if (std::find(at + 1, at + 257, (size_t)n) != at + 257) continue;
+      for (int b = 0; b < 256; ++b) at[b + 1] += at[b];
+      for (int v : ids) spare[at[key[v] >> shift & 255]++] = v;
+      ids.swap(spare);
+    }
   }
-  int axis = 0;
-  for (int c = 1; c < 3; ++c)
-    if (hi[c] - lo[c] > hi[axis] - lo[axis]) axis = c;
-  std::vector<std::pair<double, int>> key(end - begin);
-  for (size_t i = begin; i < end; ++i) key[i - begin] = {x[3 * (size_t)ids[i] + axis], ids[i]};
-  std::sort(key.begin(), key.end());
-  const int left = parts / 2;
-  const long long want = total * left / parts;
-  long long sum = 0;
-  size_t mid = begin;
-  for (size_t i = begin; i < end; ++i) {
-    ids[i] = key[i - begin].second;
-    if (sum < want) mid = i + 1;
-    sum += weight[ids[i]];
+
+  void cut(size_t begin, size_t end, int first, int parts) {
+    if (begin == end) return;
+    if (parts == 1) {
+      for (size_t i = begin; i < end; ++i) owner[order[0][i]] = first;
+      return;
+    }
+    int axis = 0;
+    double side[3];
+    for (int c = 0; c < 3; ++c) {
+      side[c] = x[3 * (size_t)order[c][end - 1] + c] - x[3 * (size_t)order[c][begin] + c];
+      if (side[c] > side[axis]) axis = c;
+    }
+    const std::vector<int>& ids = order[axis];
+    long long total = 0;
+    for (size_t i = begin; i < end; ++i) total += weight[ids[i]];
+    const int left = parts / 2;
+    const long long want = total * left / parts;
+    long long sum = 0;
+    size_t mid = begin;
+    for (; mid < end && sum < want; ++mid) sum += weight[ids[mid]];
+    // every part keeps a vertex while there are enough
+    if (end - begin >= (size_t)parts)
+      mid = std::min(std::max(mid, begin + left), end - (parts - left));
+    for (size_t i = begin; i < end; ++i) left_side[ids[i]] = i < mid;
+    for (int c = 0; c < 3; ++c) {
+      if (c == axis) continue;
+      size_t l = begin, r = mid;
+      for (size_t i = begin; i < end; ++i) {
+        const int v = order[c][i];
+        spare[left_side[v] ? l++ : r++] = v;
+      }
+      std::copy(spare.begin() + begin, spare.begin() + end, order[c].begin() + begin);
+    }
+    cut(begin, mid, first, left);
+    cut(mid, end, first + left, parts - left);
   }
-  // every part keeps a vertex while there are enough
-  if (end - begin >= (size_t)parts)
-    mid = std::min(std::max(mid, begin + left), end - (parts - left));
-  bisect(x, weight, ids, begin, mid, first, left, owner);
-  bisect(x, weight, ids, mid, end, first + left, parts - left, owner);
-}
+};
 
 // Blocks a single mesh of ns solved vertices is divided among: one per SM, down
 // to a dozen vertices a block.  fp64 us per sweep on B200 with 6 / 12 / 24 vertices
@@ -1317,10 +1343,11 @@ int domain_count(int ns, int sms) {
 // vertices 33.1 / 34.5, at 2,350: 116 / 154; 2 lanes 137).
 int domain_tpv(int n) { return n <= 16 ? 32 : (n <= 64 ? 16 : (n <= 160 ? 8 : 4)); }
 
-// Environment k in ndom domains.  X: rest positions, caller order; ltpv, tpv:
-// lanes per vertex of the solver's layout and of the domains'.
+// Environment k in ndom domains, appended to D.  X: rest positions, caller order; ltpv, tpv:
+// lanes per vertex of the solver's layout and of the domains'.  Host threads take groups of
+// domains (`groups` of them at most) and their parts are joined in order.
 void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, int ndom,
-                   bool sort_records, DomLayout& D) {
+                   bool sort_records, int groups, DomLayout& out) {
   const EnvInfo& e = L.env[k];
   const int V = e.nv, ns = e.nsolved, C = e.ncolors, cpw = 32 / tpv, lcpw = 32 / ltpv;
   const int* valence = L.valence.data() + e.vbase;
@@ -1328,18 +1355,21 @@ void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, i
   for (int v = 0; v < V; ++v)
     for (int c = 0; c < 3; ++c)
       x[3 * (size_t)(L.new_of_old[e.vbase + v] - e.vbase) + c] = X[3 * (size_t)(e.vbase + v) + c];
-  std::vector<int> owner(V, -1), ids(ns), color(ns);
-  for (int i = 0; i < ns; ++i) ids[i] = i;
-  bisect(x, valence, ids, 0, ns, 0, ndom, owner);
-  for (int c = 0; c < C; ++c)
-    for (int v = L.color[e.cbase + c].vbegin; v < L.color[e.cbase + c].vend; ++v)
+  std::vector<int> owner(V, -1), color(ns);
+  Bisection(x, valence, ns, owner).cut(0, ns, 0, ndom);
+  // the slots of vertex v in the solver's layout: slot j lies ltpv-wise in blocks of 32
+  std::vector<const int4*> slots(ns);
+  const int lshift = ltpv == 2 ? 1 : (ltpv == 4 ? 2 : (ltpv == 8 ? 3 : 4));
+  for (int c = 0; c < C; ++c) {
+    const ColorInfo& ci = L.color[e.cbase + c];
+    for (int v = ci.vbegin; v < ci.vend; ++v) {
+      const int p = v - ci.vbegin, q = ci.chunk_begin + p / lcpw;
       color[v - e.vbase] = c;
-  // the slots of vertex v in the solver's layout
+      slots[v - e.vbase] = L.rec_idx.data() + (size_t)L.chunk[q].block * 32 + p % lcpw * ltpv;
+    }
+  }
   auto slot_of = [&](int v, int j) -> const int4& {
-    const ColorInfo& ci = L.color[e.cbase + color[v]];
-    const int p = e.vbase + v - ci.vbegin;
-    const ChunkInfo& ch = L.chunk[ci.chunk_begin + p / lcpw];
-    return L.rec_idx[((size_t)ch.block + j / ltpv) * 32 + p % lcpw * ltpv + j % ltpv];
+    return slots[v][((size_t)(j >> lshift) << 5) + (j & (ltpv - 1))];
   };
   std::vector<std::vector<int>> own(ndom);
   for (int v = 0; v < ns; ++v) own[owner[v]].push_back(v);  // by colour, as numbered
@@ -1347,121 +1377,153 @@ void build_domains(const Layout& L, int ltpv, const double* X, int k, int tpv, i
   // vertices of a chunk read the same records at the same time where they can
   // (67 instead of 84 shared-memory wavefronts per 32 slots on the 160x16x16 beam,
   // with the lane order of DomChunk)
-  if (sort_records)
-    for (auto& o : own)
-      std::sort(o.begin(), o.end(), [&](int a, int b) {
-        if (color[a] != color[b]) return color[a] < color[b];
-        if (valence[a] != valence[b]) return valence[a] > valence[b];
-        for (int j = 0; j < valence[a]; ++j) {
-          const int ra = slot_of(a, j).w, rb = slot_of(b, j).w;
-          if (ra != rb) return ra < rb;
-        }
-        return a < b;
-      });
+  auto by_records = [&](int a, int b) {
+    if (color[a] != color[b]) return color[a] < color[b];
+    if (valence[a] != valence[b]) return valence[a] > valence[b];
+    for (int j = 0; j < valence[a]; ++j) {
+      const int ra = slot_of(a, j).w, rb = slot_of(b, j).w;
+      if (ra != rb) return ra < rb;
+    }
+    return a < b;
+  };
   std::vector<std::vector<int>> tets(ndom);
   for (int t = e.tbase; t < e.tbase + e.ntets; ++t) tets[owner[L.tet_owner[t]]].push_back(t);
+  struct Part {
+    DomLayout D;
+    std::vector<int> mailed;
+    bool save = true;
+  };
+  std::vector<Part> part(std::max(1, std::min(groups, ndom)));
+  const int np = (int)part.size();
+  for_each_parallel(np, [&](int g) {
+    DomLayout& D = part[g].D;
+    std::vector<int>& mailed = part[g].mailed;
+    bool& save = part[g].save;
+    const int r0 = (int)((long long)ndom * g / np), r1 = (int)((long long)ndom * (g + 1) / np);
+    std::vector<int> loc(V, -1), rec_loc(e.nrec, -1), others, recs;
+    for (int r = r0; r < r1; ++r) {
+      if (sort_records) std::sort(own[r].begin(), own[r].end(), by_records);
+      DomInfo di{};
+      di.env = k;
+      di.nd = ndom;
+      di.rank = r;
+      di.lbase = (int)D.local.size();
+      di.nown = (int)own[r].size();
+      di.tbase = (int)D.tet_slot.size();
+      di.qbase = (int)D.chunk.size();
+      di.cbase = (int)D.color.size();
+      di.ncolors = C;
+      for (int i = 0; i < di.nown; ++i) loc[own[r][i]] = i;
+      // the other vertices of its tets: solved ones by colour, then the unsolved
+      others.clear();
+      for (int v : own[r])
+        for (int j = 0; j < valence[v]; ++j) {
+          const int4& s = slot_of(v, j);
+          for (int n : {s.x, s.y, s.z})
+            if (loc[n] < 0) {
+              loc[n] = 0;
+              others.push_back(n);
+            }
+        }
+      std::sort(others.begin(), others.end());
+      for (size_t i = 0; i < others.size(); ++i) loc[others[i]] = di.nown + (int)i;
+      di.nloc = di.nown + (int)others.size();
+      for (int v : own[r]) D.local.push_back(make_int2(e.vbase + v, valence[v]));
+      for (int n : others) {
+        D.local.push_back(make_int2(e.vbase + n, 0));
+        if (n < ns) mailed.push_back(n);
+      }
+      recs.clear();
+      auto local_slot = [&](const int4& s) {
+        int& q = rec_loc[s.w >> 2];
+        if (q < 0) {
+          q = (int)recs.size();
+          recs.push_back(s.w >> 2);
+        }
+        return make_int4(loc[s.x], loc[s.y], loc[s.z], 4 * q + (s.w & 3));
+      };
+      size_t h = 0;
+      int at = 0;
+      for (int c = 0; c < C; ++c) {
+        DomColor dc{};
+        dc.chunk_begin = (int)D.chunk.size() - di.qbase;
+        int end = at;
+        while (end < di.nown && color[own[r][end]] == c) ++end;
+        for (; at < end; at += cpw) {
+          const int n = std::min(cpw, end - at);
+          int kmax = 0;
+          for (int i = 0; i < n; ++i) kmax = std::max(kmax, valence[own[r][at + i]]);
+          DomChunk ch{(int)(D.slot.size() / 32), (kmax + tpv - 1) / tpv, at, at + n};
+          D.slot.resize(D.slot.size() + 32 * (size_t)ch.steps, make_ushort4(0, 0, 0, 0));
+          ushort4* block = D.slot.data() + (size_t)ch.block * 32;
+          for (int i = 0; i < n; ++i) {
+            const int v = own[r][at + i];
+            for (int j = 0, row = 0; j < valence[v]; ++j) {
+              const int4 s = local_slot(slot_of(v, j));
+              const int lane = j - row * tpv;  // j-th slot: lane lane * cpw + i of row `row`
+              block[32 * row + lane * cpw + i] =
+                  make_ushort4((unsigned short)s.x, (unsigned short)s.y, (unsigned short)s.z,
+                               (unsigned short)s.w);
+              row += lane + 1 == tpv;
+            }
+          }
+          D.chunk.push_back(ch);
+        }
+        at = end;
+        dc.chunk_end = (int)D.chunk.size() - di.qbase;
+        dc.halo_begin = di.nown + (int)h;
+        while (h < others.size() && others[h] < ns && color[others[h]] == c) ++h;
+        dc.halo_end = di.nown + (int)h;
+        D.color.push_back(dc);
+      }
+      di.nchunk = (int)D.chunk.size() - di.qbase;
+      for (int t : tets[r]) {
+        D.tet_owner.push_back(loc[L.tet_owner[t]]);
+        D.tet_slot.push_back(local_slot(L.tet_slot[t]));
+      }
+      di.ntets = (int)tets[r].size();
+      di.nrec = (int)recs.size();
+      // shared memory: the records first, then the chunk and vertex lists
+      for (int f : {kDomRecords, kDomMeta})
+        if (dom_smem(di.nloc, di.nrec, di.nchunk, 0, di.flags | f) <= kDomMaxSmem) di.flags |= f;
+      // staged records are gathered from the environment's table; the others are read in
+      // place, so a copy in the domain's order is kept
+      if (di.flags & kDomRecords) {
+        di.rbase = (int)D.rec_id.size();
+        D.rec_id.insert(D.rec_id.end(), recs.begin(), recs.end());
+      } else {
+        di.rbase = (int)(D.rec.size() / 12);
+        for (int q : recs) {
+          const double* v = &L.table.vals[12 * (size_t)(e.rbase + q)];
+          D.rec.insert(D.rec.end(), v, v + 12);
+        }
+      }
+      while (di.nsave < di.nown && color[own[r][di.nsave]] == 0) ++di.nsave;
+      save = save && dom_smem(di.nloc, di.nrec, di.nchunk, di.nsave, di.flags | kDomSave) <=
+                         kDomMaxSmem;
+      D.fits = D.fits && dom_smem(di.nloc, 0, 0, 0, 0) <= kDomMaxSmem && di.nloc <= 65536 &&
+               di.nrec <= 65536 / 4 && C <= kDomMaxColors;
+      D.dom.push_back(di);
+      for (int v : own[r]) loc[v] = -1;
+      for (int n : others) loc[n] = -1;
+      for (int q : recs) rec_loc[q] = -1;
+      if (!D.fits) return;
+    }
+  });
   std::vector<char> mailed(ns, 0);
-  std::vector<int> loc(V, -1), rec_loc(e.nrec, -1), others, recs;
   bool save = ndom > 1;
-  for (int r = 0; r < ndom; ++r) {
-    DomInfo di{};
-    di.env = k;
-    di.nd = ndom;
-    di.rank = r;
-    di.lbase = (int)D.local.size();
-    di.nown = (int)own[r].size();
-    di.rbase = (int)(D.rec.size() / 12);
-    di.tbase = (int)D.tet_slot.size();
-    di.qbase = (int)D.chunk.size();
-    di.cbase = (int)D.color.size();
-    di.ncolors = C;
-    for (int i = 0; i < di.nown; ++i) loc[own[r][i]] = i;
-    // the other vertices of its tets: solved ones by colour, then the unsolved
-    others.clear();
-    for (int v : own[r])
-      for (int j = 0; j < valence[v]; ++j) {
-        const int4& s = slot_of(v, j);
-        for (int n : {s.x, s.y, s.z})
-          if (loc[n] < 0) {
-            loc[n] = 0;
-            others.push_back(n);
-          }
-      }
-    std::sort(others.begin(), others.end());
-    for (size_t i = 0; i < others.size(); ++i) loc[others[i]] = di.nown + (int)i;
-    di.nloc = di.nown + (int)others.size();
-    for (int v : own[r]) D.local.push_back(make_int2(e.vbase + v, valence[v]));
-    for (int n : others) {
-      D.local.push_back(make_int2(e.vbase + n, 0));
-      if (n < ns) mailed[n] = 1;
-    }
-    recs.clear();
-    auto local_slot = [&](const int4& s) {
-      int& q = rec_loc[s.w >> 2];
-      if (q < 0) {
-        q = (int)recs.size();
-        recs.push_back(s.w >> 2);
-      }
-      return make_int4(loc[s.x], loc[s.y], loc[s.z], 4 * q + (s.w & 3));
-    };
-    size_t h = 0;
-    int at = 0;
-    for (int c = 0; c < C; ++c) {
-      DomColor dc{};
-      dc.chunk_begin = (int)D.chunk.size() - di.qbase;
-      int end = at;
-      while (end < di.nown && color[own[r][end]] == c) ++end;
-      for (; at < end; at += cpw) {
-        const int n = std::min(cpw, end - at);
-        int kmax = 0;
-        for (int i = 0; i < n; ++i) kmax = std::max(kmax, valence[own[r][at + i]]);
-        DomChunk ch{(int)(D.slot.size() / 32), (kmax + tpv - 1) / tpv, at, at + n};
-        D.slot.resize(D.slot.size() + 32 * (size_t)ch.steps, make_ushort4(0, 0, 0, 0));
-        for (int i = 0; i < n; ++i)
-          for (int j = 0; j < valence[own[r][at + i]]; ++j) {
-            const int4 s = local_slot(slot_of(own[r][at + i], j));
-            D.slot[((size_t)ch.block + j / tpv) * 32 + j % tpv * cpw + i] =
-                make_ushort4((unsigned short)s.x, (unsigned short)s.y, (unsigned short)s.z,
-                             (unsigned short)s.w);
-          }
-        D.chunk.push_back(ch);
-      }
-      at = end;
-      dc.chunk_end = (int)D.chunk.size() - di.qbase;
-      dc.halo_begin = di.nown + (int)h;
-      while (h < others.size() && others[h] < ns && color[others[h]] == c) ++h;
-      dc.halo_end = di.nown + (int)h;
-      D.color.push_back(dc);
-    }
-    di.nchunk = (int)D.chunk.size() - di.qbase;
-    for (int t : tets[r]) {
-      D.tet_owner.push_back(loc[L.tet_owner[t]]);
-      D.tet_slot.push_back(local_slot(L.tet_slot[t]));
-    }
-    di.ntets = (int)tets[r].size();
-    di.nrec = (int)recs.size();
-    for (int q : recs) {
-      const double* v = &L.table.vals[12 * (size_t)(e.rbase + q)];
-      D.rec.insert(D.rec.end(), v, v + 12);
-    }
-    // shared memory: the records first, then the chunk and vertex lists
-    for (int f : {kDomRecords, kDomMeta})
-      if (dom_smem(di.nloc, di.nrec, di.nchunk, 0, di.flags | f) <= kDomMaxSmem) di.flags |= f;
-    while (di.nsave < di.nown && color[own[r][di.nsave]] == 0) ++di.nsave;
-    save = save && dom_smem(di.nloc, di.nrec, di.nchunk, di.nsave, di.flags | kDomSave) <=
-                       kDomMaxSmem;
-    D.fits = D.fits && dom_smem(di.nloc, 0, 0, 0, 0) <= kDomMaxSmem && di.nloc <= 65536 &&
-             di.nrec <= 65536 / 4 && C <= kDomMaxColors;
-    D.dom.push_back(di);
-    for (int v : own[r]) loc[v] = -1;
-    for (int n : others) loc[n] = -1;
-    for (int q : recs) rec_loc[q] = -1;
-    if (!D.fits) return;
+  for (Part& p : part) {
+    save = save && p.save;
+    for (int n : p.mailed) mailed[n] = 1;
   }
-  for (DomInfo& di : D.dom) {
-    if (save) di.flags |= kDomSave;
-    for (int l = di.lbase; l < di.lbase + di.nown; ++l)
-      if (mailed[D.local[l].x - e.vbase]) D.local[l].x = ~D.local[l].x;
+  for (Part& p : part) {
+    for (DomInfo& di : p.D.dom) {
+      if (save) di.flags |= kDomSave;
+      for (int l = di.lbase; l < di.lbase + di.nown; ++l)
+        if (mailed[p.D.local[l].x - e.vbase]) p.D.local[l].x = ~p.D.local[l].x;
+    }
+    out.append(p.D);
+    p.D = DomLayout();
   }
 }
 
@@ -1473,7 +1535,8 @@ void build_all_domains(const Layout& L, int ltpv, const double* X, int tpv, int 
   const int n = (int)L.env.size();
   std::vector<DomLayout> each(n);
   for_each_parallel(n, [&](int k) {
-    build_domains(L, ltpv, X, k, tpv, parts, sort_records, each[k]);
+    build_domains(L, ltpv, X, k, tpv, parts, sort_records, n == 1 ? L.env[0].nsolved / 256 : 1,
+                  each[k]);
   });
   first.resize(n);
   smem.assign(n, 0);
@@ -1488,17 +1551,7 @@ void build_all_domains(const Layout& L, int ltpv, const double* X, int tpv, int 
 
 // The next step's number (vbd_domain.h: tags), and the arrays of a launch.
 DomDev dom_dev(const vbd_solver* s) {
-  DomDev d{};
-  d.dom = s->d_dom.p;
-  d.color = s->d_dom_color.p;
-  d.chunk = s->d_dom_chunk.p;
-  d.slot = s->d_dom_slot.p;
-  d.local = s->d_dom_local.p;
-  d.rec = reinterpret_cast<const double4*>(s->d_dom_rec.p);
-  d.tet_slot = s->d_dom_tet.p;
-  d.tet_owner = s->d_dom_tet_owner.p;
-  d.mail = s->d_dom_mail.p;
-  d.post = s->d_dom_post.p;
+  DomDev d = s->dom;
   d.abort = s->d_status.p + s->n_env;
   d.seq = s->dom_seq;
   d.grid_sync = (s->flags & VBD_PERSIST_GRID_BARRIERS) ? 1 : 0;
@@ -1531,8 +1584,8 @@ cudaError_t launch_block(const vbd_solver* s, const DevMesh& m, const StepParams
                            cluster, smem, st);
   DomDev d = dom_dev(s);
   d.work = work;
-  d.first_single = s->d_dom_first[0].p;
-  d.first_split = s->d_dom_first[cluster == s->cluster ? 1 : 2].p;
+  d.first_single = s->dom_first[0];
+  d.first_split = s->dom_first[cluster == s->cluster ? 1 : 2];
   return launch_domain(s->material, s->dom_tpv, threads, m, p, d, tol, s->wait_limits, n_blocks,
                        cluster, false, smem, st);
 }
@@ -1875,24 +1928,61 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
         di.pbase = posts - 2 * di.nd;
         split = split || di.nd > 1;
       }
-      for (int i = 0; i < 3 && !err; ++i)
-        if (parts[i] > 0 && bad(s->d_dom_first[i].upload(first[i], st), "domains")) err = 1;
-      if (err || bad(s->d_dom.upload(D.dom, st), "domains") ||
-          bad(s->d_dom_color.upload(D.color, st), "domains") ||
-          bad(s->d_dom_chunk.upload(D.chunk, st), "domains") ||
-          bad(s->d_dom_slot.upload(D.slot, st), "domains") ||
-          bad(s->d_dom_local.upload(D.local, st), "domains") ||
-          bad(s->d_dom_rec.upload(D.rec, st), "domains") ||
-          bad(s->d_dom_tet.upload(D.tet_slot, st), "domains") ||
-          bad(s->d_dom_tet_owner.upload(D.tet_owner, st), "domains") ||
-          bad(s->d_dom_mail.alloc(split ? 3 * (size_t)V : 1), "domains") ||
-          bad(s->d_dom_post.alloc((size_t)posts), "domains") ||
-          bad(cudaMemsetAsync(s->d_dom_mail.p, 0, sizeof(ulonglong2) * s->d_dom_mail.n, st),
-              "domains") ||
-          bad(cudaMemsetAsync(s->d_dom_post.p, 0, sizeof(ulonglong2) * s->d_dom_post.n, st),
-              "domains"))
+      // one allocation for all arrays; the last two start at zero
+      struct Piece {
+        const void* from;
+        size_t bytes, at;
+      };
+      std::vector<Piece> pieces;
+      size_t total = 0;
+      auto place = [&](const void* from, size_t bytes) {
+        pieces.push_back({from, bytes, total});
+        total += (bytes + 255) / 256 * 256;
+        return pieces.back().at;
+      };
+      auto array = [&](const auto& v) { return place(v.data(), v.size() * sizeof(v[0])); };
+      size_t at_first[3] = {0, 0, 0};
+      for (int i = 0; i < 3; ++i) at_first[i] = array(first[i]);
+      const size_t at_dom = array(D.dom), at_color = array(D.color), at_chunk = array(D.chunk),
+                   at_slot = array(D.slot), at_local = array(D.local),
+                   at_id = array(D.rec_id), at_rec = array(D.rec),
+                   at_tet = array(D.tet_slot), at_owner = array(D.tet_owner), filled = total;
+      const size_t at_mail = place(nullptr, sizeof(ulonglong2) * (split ? 3 * (size_t)V : 1));
+      const size_t at_post = place(nullptr, sizeof(ulonglong2) * (size_t)posts);
+      std::vector<unsigned char> together;  // small ones in one copy
+      if (bad(s->d_dom.alloc(total), "domains")) {
         err = 1;
-      cudaStreamSynchronize(st);  // D and first go out of scope
+      } else if (filled <= ((size_t)1 << 20)) {
+        together.resize(filled);
+        for (const Piece& q : pieces)
+          if (q.from && q.bytes) std::memcpy(together.data() + q.at, q.from, q.bytes);
+        if (bad(cudaMemcpyAsync(s->d_dom.p, together.data(), filled, cudaMemcpyHostToDevice, st),
+                "domains"))
+          err = 1;
+      } else {
+        for (const Piece& q : pieces)
+          if (!err && q.from && q.bytes &&
+              bad(cudaMemcpyAsync(s->d_dom.p + q.at, q.from, q.bytes, cudaMemcpyHostToDevice, st),
+                  "domains"))
+            err = 1;
+      }
+      if (!err && bad(cudaMemsetAsync(s->d_dom.p + filled, 0, total - filled, st), "domains"))
+        err = 1;
+      cudaStreamSynchronize(st);  // the host arrays go out of scope
+      unsigned char* base = s->d_dom.p;
+      for (int i = 0; i < 3; ++i)
+        s->dom_first[i] = reinterpret_cast<const int*>(base + at_first[i]);
+      s->dom.dom = reinterpret_cast<const DomInfo*>(base + at_dom);
+      s->dom.color = reinterpret_cast<const DomColor*>(base + at_color);
+      s->dom.chunk = reinterpret_cast<const DomChunk*>(base + at_chunk);
+      s->dom.slot = reinterpret_cast<const ushort4*>(base + at_slot);
+      s->dom.local = reinterpret_cast<const int2*>(base + at_local);
+      s->dom.rec_id = reinterpret_cast<const int*>(base + at_id);
+      s->dom.rec = reinterpret_cast<const double4*>(base + at_rec);
+      s->dom.tet_slot = reinterpret_cast<const int4*>(base + at_tet);
+      s->dom.tet_owner = reinterpret_cast<const int*>(base + at_owner);
+      s->dom.mail = reinterpret_cast<ulonglong2*>(base + at_mail);
+      s->dom.post = reinterpret_cast<ulonglong2*>(base + at_post);
       s->sms = sms;
       for (int i = 0; i < 3; ++i)
         for (size_t e = 0; e < first[i].size(); ++e) {
@@ -2057,10 +2147,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
   s->device_bytes += (long long)(4 * sb + s->d_X.n * 8 + s->d_io.n * 8);
   s->device_bytes += (long long)(s->d_valence.n * 4 + s->d_map.n * 4);
   s->device_bytes += (long long)(s->d_tet_slot.n * sizeof(int4) + s->d_tet_owner.n * 4);
-  auto bytes = [](const auto&... b) { return (long long)((b.n * sizeof(*b.p)) + ...); };
-  s->device_bytes += bytes(s->d_dom, s->d_dom_color, s->d_dom_chunk, s->d_dom_slot, s->d_dom_local,
-                           s->d_dom_rec, s->d_dom_tet, s->d_dom_tet_owner, s->d_dom_mail,
-                           s->d_dom_post, s->d_dom_first[0], s->d_dom_first[1], s->d_dom_first[2]);
+  s->device_bytes += (long long)s->d_dom.n;
   *out = s;
   return VBD_OK;
 }
