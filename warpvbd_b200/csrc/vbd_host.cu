@@ -12,15 +12,11 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <exception>
 #include <mutex>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -30,6 +26,7 @@
 #include "vbd_domain.h"
 #include "vbd_persist.h"
 #include "vbd_noalloc.h"
+#include "vbd_parallel.h"
 #include "vbd_plan.h"
 #include "vbd_setup.h"
 #include "vbd_warmstart.h"
@@ -103,36 +100,6 @@ int greedy_coloring(const int32_t* tets, int T, int nv, int32_t* col) {
     ncol = std::max(ncol, c + 1);
   }
   return ncol;
-}
-
-// f(0) ... f(n - 1) on up to 16 host threads; an exception of f is rethrown here.
-template <class F>
-void for_each_parallel(int n, F f) {
-  std::atomic<int> next{0};
-  std::mutex mu;
-  std::exception_ptr error;
-  auto work = [&]() {
-    for (int k; (k = next.fetch_add(1)) < n;) {
-      try {
-        f(k);
-      } catch (...) {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!error) error = std::current_exception();
-        next = n;
-      }
-    }
-  };
-  const int nthreads =
-      std::min<int>(n, std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
-  std::vector<std::thread> pool;
-  pool.reserve(nthreads);
-  try {
-    for (int i = 1; i < nthreads; ++i) pool.emplace_back(work);
-  } catch (const std::system_error&) {  // no more threads: those there are do it
-  }
-  work();
-  for (auto& t : pool) t.join();
-  if (error) std::rethrow_exception(error);
 }
 
 struct TetData {
