@@ -23,3 +23,27 @@ def test_forward_tiles(n, offset):
     ref = ref[0] if isinstance(ref, tuple) else ref
     # three layers of at most 64 fp32 roundings (2^-24 each) of values of the result's size
     assert np.abs(out - ref).max() < 3 * 64 * 2.0 ** -24 * max(1.0, np.abs(ref).max())
+
+
+def test_forward_from_several_threads():
+    """First calls of both tile sizes at once, a thread and a stream each."""
+    import threading
+    import torch
+    p = ws.init_params(2)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    X = [torch.randn(148 * 256 + 64 if k % 2 else 1000, ws.FEAT_WIDTH, device="cuda", generator=g)
+         for k in range(8)]
+    torch.cuda.synchronize()
+    out = [None] * 8
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            out[k] = ws.MLPTrainer(p, max_batch=64).forward(X[k])  # its stream: this one
+            torch.cuda.current_stream().synchronize()
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(8):
+        assert torch.equal(out[k], ws.MLPTrainer(p, max_batch=64).forward(X[k]))

@@ -700,7 +700,8 @@ cudaError_t dom_dispatch(int material, int tpv, bool split, F& f) {
 
 template <int TPV, int MAT, bool SPLIT>
 cudaError_t dom_configure() {
-  static int configured_device = -1;  // the attributes are per device
+  // the attributes are per device; each thread sets them for itself
+  static thread_local int configured_device = -1;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_device == dev) return cudaSuccess;

@@ -730,8 +730,10 @@ cudaError_t launch_mlp_train_batch(const float* X, const float* Y, const int* id
 
 namespace {
 template <int SPT>
-cudaError_t forward_tiles(const float* X, int n, const float* P, float* out, cudaStream_t s) {
-  static int configured_device = -1, per_sm = 0, sms = 0;  // the attributes are per device
+cudaError_t forward_tiles(const float* X, int n, const float* P, float* out, int sms,
+                          cudaStream_t s) {
+  // the attributes are per device; each thread sets them for itself
+  static thread_local int configured_device = -1, per_sm = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_device != dev) {
@@ -741,7 +743,6 @@ cudaError_t forward_tiles(const float* X, int n, const float* P, float* out, cud
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mlp_forward_kernel<SPT>,
                                                         kFwdThreads, kFwSmem<SPT>);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     configured_device = dev;
   }
@@ -754,10 +755,18 @@ cudaError_t forward_tiles(const float* X, int n, const float* P, float* out, cud
 cudaError_t launch_mlp_forward(const float* X, int n, const float* P, float* out,
                                cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  // 128-sample tiles reuse the weights more; below one wave of them, 64-sample
+  static thread_local int known_device = -1, sms = 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (known_device != dev) {
+    const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    known_device = dev;
+  }
+  // 128-sample tiles reuse the weights more; below one wave of them (two a SM), 64-sample
   // tiles fill the device better
-  return n >= 148 * 2 * 128 ? forward_tiles<8>(X, n, P, out, s)
-                            : forward_tiles<4>(X, n, P, out, s);
+  return n >= sms * 2 * 128 ? forward_tiles<8>(X, n, P, out, sms, s)
+                            : forward_tiles<4>(X, n, P, out, sms, s);
 }
 
 cudaError_t launch_adam(float* P, const float* G, float* M, float* V, int n, float lr,
