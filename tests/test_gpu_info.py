@@ -39,3 +39,13 @@ def test_tuner_reaches_the_automatic_shape(tmp_path):
     auto, ran = (VBDSolver(**kw, **KW, damping_coefficient=0.0, **c).info() for c in ({}, cfg))
     assert auto["mode"] == ran["mode"] == 0x400 and auto["tpv"] == 32
     assert cfg["block_threads"] == ran["block_threads"] and cfg["tpv"] in (0, ran["tpv"])
+
+
+def test_two_lanes_asked_for_take_twice_the_threads():
+    kw = dict(scenes.cantilever(20).solver_kwargs(), **KW, damping_coefficient=0.0, mode="block",
+              cluster=1)
+    for tpv, threads, ran in ((2, 128, 256), (2, 512, 512), (4, 128, 128), (2, 0, 512)):
+        info = VBDSolver(**kw, tpv=tpv, block_threads=threads).info()
+        assert info["tpv"] == 4 and info["block_threads"] == ran
+    mixed = VBDSolver(**kw, precision="mixed", tpv=2, block_threads=128).info()
+    assert mixed["tpv"] == 2 and mixed["block_threads"] == 128
