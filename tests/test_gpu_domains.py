@@ -254,6 +254,10 @@ def test_default_thread_count_of_a_batch(cube, n, threads):
     envs = [scenes.mass_spring(cube, 3)] * n
     sol = BatchedVBDSolver(envs, dx_tol=1e-7, max_iter=1000, cluster=1)
     assert sol.info()["block_threads"] == threads
+    asked = BatchedVBDSolver(envs[:4], dx_tol=1e-7, max_iter=1000, cluster=1, block_threads=512)
+    assert asked.info()["block_threads"] == {2: 128, 5: 256, 7: 512, 15: 512}[cube]
+    asked = BatchedVBDSolver(envs[:4], dx_tol=1e-7, max_iter=1000, cluster=1, block_threads=64)
+    assert asked.info()["block_threads"] == (512 if cube == 15 else 64)
     its, x = _steps(sol, 2)
     ref = BatchedVBDSolver(envs[:1], dx_tol=1e-7, max_iter=1000, cluster=1, tpv=4,
                            block_threads=64)

@@ -1206,7 +1206,9 @@ struct DomLayout {
 // vertices (4 chunks) 445 / 423 / 432, 100 of 225 (6) 425 / 339 / 349, 100 of 350 (9) 556 /
 // 428 / 374; 300 of 225 472 / 496 / 717, 300 of 350 651 / 589 / 734, 1,000 of 40 883 / 1683 /
 // 2935.
-int single_threads(const DomLayout& D, int n_env, int sms) {
+// asked: a count the caller gave, of which no more are launched than have a chunk (1,000
+// environments of 95 vertices, 512 threads asked for: 3370 -> 1088; 128 run).
+int single_threads(const DomLayout& D, int n_env, int sms, int asked) {
   int most = 1;
   for (const DomInfo& di : D.dom)
     if (di.nd == 1)
@@ -1214,6 +1216,7 @@ int single_threads(const DomLayout& D, int n_env, int sms) {
         most = std::max(most, D.color[c].chunk_end - D.color[c].chunk_begin);
   int threads = 128;
   while (threads < kDomMaxThreads && threads < 32 * most) threads *= 2;
+  if (asked) return std::min(asked, threads);
   return n_env > sms ? std::min(threads, 256) : threads;
 }
 
@@ -1972,7 +1975,7 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
         // blocks too large for two on an SM get the SM's warps
         auto fills_sm = [](size_t x) { return 2 * (x + 7 * 1024) > 227 * 1024; };
         s->split_threads = fills_sm(s->smem_bytes) ? kDomMaxThreads : s->threads;
-        if (!threads_arg && s->n_env > 1) s->threads = single_threads(D, s->n_env, sms);
+        if (s->n_env > 1) s->threads = single_threads(D, s->n_env, sms, threads_arg);
         if (fills_sm(s->n_env > 1 ? s->smem_single : s->smem_bytes)) s->threads = kDomMaxThreads;
       }
     } else if (block_mode && s->n_env > 1) {
