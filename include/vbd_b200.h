@@ -171,7 +171,8 @@ int vbd_set_wait_limits(vbd_solver* s, long long max_polls, unsigned long long m
  * (blocks without an environment, padding a cluster, leave zeros).
  * vbd_get_trace copies the last finished step's records, at most `cap`, and
  * writes their number to *count (records = NULL: only the number); the other
- * modes record nothing (count 0). */
+ * modes record nothing (count 0), except that a small mesh (one that block mode
+ * would hold) records its domains when the automatic mode runs it in persistent mode. */
 int vbd_set_trace(vbd_solver* s, int enable);
 int vbd_get_trace(vbd_solver* s, unsigned long long* records, int cap, int* count);
 
@@ -183,7 +184,8 @@ int vbd_reset(vbd_solver* s);
  * max_iter sweeps, then v = (x_new - x_old)/dt.  With iterations_out != NULL
  * the call blocks and writes the sweep count (per environment for the batched
  * form); with NULL it only enqueues the work on the solver's stream.
- * tol_per_env (batched only) may be NULL to use tol everywhere. */
+ * tol_per_env (batched only; block mode, or the automatic mode on a mesh that block mode
+ * would hold) may be NULL to use tol everywhere. */
 int vbd_step(vbd_solver* s, double dt, double tol, int max_iter, int* iterations_out);
 int vbd_step_batched(vbd_solver* s, double dt, double tol, const double* tol_per_env,
                      int max_iter, int* iterations_out);
@@ -191,7 +193,7 @@ int vbd_step_batched(vbd_solver* s, double dt, double tol, const double* tol_per
  * reference drivers read every step's positions: run_mass_spring_parallel.py
  * and run_cantilever.py:156).  When positions_out is page-locked, device-mapped
  * host memory (cudaHostAlloc / cudaMallocHost, or torch pin_memory) and the
- * solver runs in block mode, each environment's block writes its final
+ * solver runs in block mode (or as for tol_per_env above), each environment's block writes its final
  * positions there directly as it finishes, overlapping the transfer with the
  * environments still running; otherwise the positions are copied after the
  * step.  The values are the same either way. */

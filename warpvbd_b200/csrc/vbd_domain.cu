@@ -322,7 +322,9 @@ __global__ void __launch_bounds__(kDomMaxThreads)
     unsigned char* stab = dsmem + dom_smem_records(di.nloc);
     tab = global_table<double>(m.rec_tab, e.rbase);
     const int* id = d.rec_id + di.rbase;
-    stage_rows(stab, di.nrec, [&](int rec, int row) { return tab.g + 3 * (size_t)__ldg(id + rec) + row; });
+    stage_rows(stab, di.nrec, [&](int rec, int row) {
+      return tab.g + 3 * (size_t)__ldg(id + rec) + row;
+    });
     tab = staged(tab, stab);
   }
   const int4* chunk = reinterpret_cast<const int4*>(d.chunk) + di.qbase;
