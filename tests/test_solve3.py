@@ -1,6 +1,7 @@
 """The fp64 3x3 solve and the reciprocal of the vertex update (warpvbd_b200/csrc/vbd_solve.h),
-compiled for the host, against exact rational arithmetic: blocks of well-shaped tets, of nearly incompressible
-ones (one stiff direction, lambda / mu up to 1e12) and of very different scales."""
+compiled for the host, against exact rational arithmetic: blocks of well-shaped tets, of
+nearly incompressible ones (one stiff direction, lambda / mu up to 1e12) and of very different
+scales."""
 import ctypes
 import os
 import subprocess
@@ -59,12 +60,14 @@ def _packed(H):
     return H[np.triu_indices(3)]
 
 
-@pytest.mark.parametrize("scale", [1.0, 1e-100, 1e100])
+@pytest.mark.parametrize("scale", [1.0, 1e-63, 1e-62, 1e62, 1e63, 1e-100, 1e100])
 @pytest.mark.parametrize("k", [0.0, 1.0, 1e3, 1e5, 1e7, 1e9, 1e12])
 def test_error_grows_with_the_condition_number_only(solve3, k, scale):
     """A backward-stable factorisation of a 3x3 positive definite matrix solves H + dH with
     |dH| <= (3n + 1) u |L| |D| |L^T| (Higham, Accuracy and Stability of Numerical Algorithms,
-    10.1): a relative error of at most 3 (3n + 1) u cond(H) = 30 u cond(H) in the norm."""
+    10.1): a relative error of at most 3 (3n + 1) u cond(H) = 30 u cond(H) in the norm.  The
+    elimination step with Cramer's rule on what is left keeps within it; from scales of
+    1e-62 and 1e62 on its products leave the range and L D L^T is taken."""
     rng = np.random.default_rng(int(np.log10(k + 1)))
     for _ in range(60):
         c, M, g = rng.standard_normal(3), rng.standard_normal((3, 3)), rng.standard_normal(3)

@@ -283,14 +283,7 @@ __device__ __forceinline__ TetRows load_rows(const RecTab<double>& t, int w) {
 
 // The fp64 vertex update is written with explicit fused multiply-adds: which
 // product of a sum the compiler fuses may differ between two kernels, and every
-// launch shape has to give an environment the same bits.
-__device__ __forceinline__ double dot3(double a0, double b0, double a1, double b1, double a2,
-                                       double b2) {
-  return fma(a2, b2, fma(a1, b1, a0 * b0));
-}
-__device__ __forceinline__ double cross2(double a, double b, double c, double d) {  // ab - cd
-  return fma(a, b, -(c * d));
-}
+// launch shape has to give an environment the same bits (dot3, cross2, solve3: vbd_solve.h).
 
 // Displacement gradient of an fp64 slot: uo the vertex's own displacement,
 // n0, n1, n2 its neighbours'.
@@ -312,15 +305,6 @@ __device__ __forceinline__ void slot_gradient64(const double4& uo, const double4
   G[6] = dot3(d0z, t.r0.x, d1z, t.r1.x, d2z, t.r2.x);
   G[7] = dot3(d0z, t.r0.y, d1z, t.r1.y, d2z, t.r2.y);
   G[8] = dot3(d0z, t.r0.z, d1z, t.r1.z, d2z, t.r2.z);
-}
-
-// 1 / x for 1 <= x < 2^1022: the hardware's approximation and newton_reciprocal.  The IEEE
-// divide gives the same bits in five of six timed cases (1.2e-15 apart in the sixth) and
-// takes up to 2 % more of a step.
-__device__ __forceinline__ double reciprocal64(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  return newton_reciprocal(x, y);
 }
 
 // As slot_accumulate, in fp64; the multiples of the identity in the Hessian
@@ -363,6 +347,8 @@ __device__ __forceinline__ void slot_accumulate64(const double4& uo, const doubl
     const double Cbx = fma(bx, cx, cross2(F10, wz, F20, wy));
     const double Cby = fma(bx, cy, cross2(F20, wx, F00, wz));
     const double Cbz = fma(bx, cz, cross2(F00, wy, F10, wx));
+    // Ic + 1 >= 1.  The IEEE divide gives the same bits in five of six timed cases (1.2e-15
+    // apart in the sixth) and takes up to 2 % more of a step
     const double inv = reciprocal64(Ic + 1.0);
     const double ka = t.p0 * (1.0 - inv);
     const double kJ = fma(t.p1, J - 1.0, -0.75 * t.p0);
