@@ -40,7 +40,7 @@
 // acquire polling).  From about 300 vertices a domain the fp64 pipe and the
 // shared-memory pipe, each about half busy.  B200, fp64, us per sweep, positions
 // in global memory and flags between blocks (vbd_persist.cu) -> here: 80x8x8 StVK
-// beam 37.7 -> 17.0, 160x16x16 beam 48.8 -> 31.5, 320x32x32 beam 178 -> 117.
+// beam 38.1 -> 17.9, 160x16x16 beam 49.1 -> 30.9, 320x32x32 beam 179 -> 121.
 // Tried: reading a slot's operands while the previous slot is computed (231
 // registers, 8 warps: 35.2 and 137 us on the two larger beams), slots in pairs (no
 // change), 16 lanes per vertex on the large ones (42 us at 160x16x16).

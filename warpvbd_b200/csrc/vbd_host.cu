@@ -1633,8 +1633,8 @@ int create_impl(const double* X, int V, const int32_t* tets, int T, const double
     // or one cluster, holding the mesh in shared memory wins up to ~2k vertices;
     // beyond that the persistent kernel over the whole GPU.  In fp64 the
     // persistent step by domains wins from a few dozen vertices on (us per sweep,
-    // one block or cluster -> domains: 189 vertices 18.9 -> 13.7, 1,025 vertices
-    // 41 -> 15, 1,808 vertices 44 -> 19).
+    // one block or cluster -> domains: 189 vertices 18.9 -> 13.4, 1,025 vertices
+    // 34 -> 13.5, 1,808 vertices 44 -> 16.6).
     // A cluster size asked for is block mode's.
     const bool holds = fits && V <= 2048;
     if (s->n_env > 1 || (holds && (!s->fp64 || V <= 96 || cl)))

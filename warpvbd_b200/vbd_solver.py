@@ -163,10 +163,12 @@ class VBDSolver:
                  steps and 9.6e-5 on the 256-environment batch) or "fp32"
                  (everything fp32)
       mode       "auto", "block", "graph", "hostloop" or "persist" (see include/vbd_b200.h)
-      tpv, block_threads   launch shape (0 = automatic; in fp64 the persistent mode
-                 takes its own thread count)
+      tpv, block_threads   launch shape (0 = automatic; in fp64 at least 4 lanes run, the
+                 persistent mode takes its own thread count, and 2 lanes asked for
+                 double a count given; info() names what is launched)
       cluster    block mode: spread the mesh over this many thread blocks of one
-                 cluster (1 to 16; 0 = automatic)
+                 cluster (1 to 16; 0 = automatic); selects block mode under "auto" for
+                 meshes it holds
       order_index  keep ascending vertex index inside a colour (default: by valence)
       tune       pick mode / tpv / block_threads / cluster / order_index with the
                  autotuner (warpvbd_b200.autotune; measured once per mesh and GPU
