@@ -56,6 +56,11 @@ inline int split_count(const std::vector<double>& d1, const std::vector<double>&
   double best_t = launch_time(d1, dC, 0, C, clusters, sms);
   for (int h : {bound, together, n}) {
     if (h <= 0) continue;
+    // at least its jobs' total over the places: most counts end here, without a simulation
+    double total = 0.0;
+    for (int i = 0; i < h; ++i) total += dC[i];
+    for (int i = h; i < n; i += C) total += d1[i];
+    if (total >= best_t * clusters) continue;
     const double t = launch_time(d1, dC, h, C, clusters, sms);
     if (t < best_t * 0.999) {
       best_t = t;
