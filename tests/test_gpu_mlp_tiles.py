@@ -47,3 +47,31 @@ def test_forward_from_several_threads():
         t.join()
     for k in range(8):
         assert torch.equal(out[k], ws.MLPTrainer(p, max_batch=64).forward(X[k]))
+
+
+def test_training_step_under_capture():
+    """Gradient and Adam update captured in a graph and replayed: the bits of the eager calls
+    (the reduction and the update are launched before the kernel ahead of them has ended)."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(5)
+    X = torch.randn(1000, ws.FEAT_WIDTH, device="cuda", generator=g)
+    Y = torch.randn(1000, ws.N_OUT, device="cuda", generator=g)
+    idx = torch.randperm(1000, device="cuda", generator=g).to(torch.int32)
+    p = ws.init_params(4)
+    ref = ws.MLPTrainer(p, max_batch=1024)
+    grad, loss = ref.gradient(X, Y, idx)
+    grad, loss = grad.clone(), loss.clone()
+    ref.step(2e-3)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        tr = ws.MLPTrainer(p, max_batch=1024)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        out = tr.gradient(X, Y, idx)
+        tr.step(2e-3)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], grad) and torch.equal(out[1], loss)
+    assert torch.equal(tr.P, ref.P)
